@@ -219,7 +219,8 @@ def prepare(case, seed):
         mu = _directions(g, 32)
         dt = TORCH[case["dtype"]]
         p = _catalogue(g, case["n"], mu).to(dt)
-        return dict(case=case, tree=kb.GpuTree.build(p), q=_catalogue(g, case["nq"], mu).to(dt))
+        return dict(case=case, tree=kb.GpuTree.build(p), q=_catalogue(g, case["nq"], mu).to(dt),
+                    room=_room(case))
     if kind == "forest":
         sizes = _split(case["n"], case["trees"], 10_000, 100.0)
         per = torch.bincount(torch.randint(0, case["trees"], (case["nq"],), generator=g,
@@ -232,7 +233,7 @@ def prepare(case, seed):
             of.append(torch.full((per[t],), t, dtype=torch.int32, device="cuda"))
         chord = torch.exp(math.log(1e-4) + _rand(g, case["nq"]) * math.log(100.0))
         return dict(case=case, forest=kb.Forest(trees), q=torch.cat(qs), of=torch.cat(of),
-                    radii=(chord * chord).to(torch.float32))
+                    radii=(chord * chord).to(torch.float32), room=_room(case))
     # chamfer: source clouds spread over a factor of 20, targets 4x as many
     trees, src, tgt, of, base, at = [], [], [], [], [], 0
     for t, n in enumerate(_split(case["n_src"], case["pairs"], 1000, 20.0)):
@@ -254,6 +255,19 @@ def _fields(r):
     return {k: v for k, v in r.__dict__.items() if v is not None}
 
 
+def _static(r, room):
+    """A radius result in buffers of a fixed size, zeros after the hits: what a
+    program with static shapes hands on."""
+    pad = (0, max(0, room - r.distances.shape[0]))
+    return {"offsets": r.offsets, "distances": torch.nn.functional.pad(r.distances, pad),
+            "items": torch.nn.functional.pad(r.items, pad)}
+
+
+def _room(case):
+    """Hits to make room for: well above what such a batch finds."""
+    return int(2.5 * case["nq"] * _mean_hits(case)) + 20_000
+
+
 def run(s):
     c = s["case"]
     kind = c["kind"]
@@ -269,14 +283,15 @@ def run(s):
              .nearest_n(kb.SquaredEuclidean, c["k"]).within(c["radius"]).execute_gpu())
     elif kind == "within":
         b = s["tree"].query(s["q"]).within(kb.SquaredEuclidean, c["chord"] ** 2)
-        r = (b if c["sort"] else b.unsorted()).execute_gpu()
+        return _static((b if c["sort"] else b.unsorted()).execute_gpu(), s["room"])
     elif kind == "forest":
         b = s["forest"].query(s["q"], s["of"], s["radii"])
         if c["family"] == "best":
             r = b.best_n_within(kb.SquaredEuclidean, 0.0, 5).execute_gpu()
         else:
             b = b.within(kb.SquaredEuclidean, 0.0)
-            r = (b if c["family"] == "within" else b.unsorted()).execute_gpu()
+            return _static((b if c["family"] == "within" else b.unsorted()).execute_gpu(),
+                           s["room"])
     elif kind == "chamfer":
         loss, ctx = chamfer.chamfer_forward(s["forest"], s["src"], s["tgt"], c["k"], 0.01,
                                             s["of"], s["base"])
@@ -294,6 +309,15 @@ def _hits(n, chord):
     return 0.7 * n * chord * chord / 4 + 0.3 * (0.3 * n / 32) * (1 - math.exp(-chord * chord / 4e-5))
 
 
+def _mean_hits(case):
+    if case["kind"] == "within":
+        return _hits(case["n"], case["chord"])
+    # log-uniform radii over trees of geometric sizes: a mean over both
+    sizes = _split(case["n"], case["trees"], 10_000, 100.0)
+    chords = [1e-4 * 100 ** ((i + 0.5) / 16) for i in range(16)]
+    return sum(_hits(m, r) for m in sizes for r in chords) / (len(sizes) * len(chords))
+
+
 def work(case):
     """Queries in, results out, and the entries the answers come from: one
     32-entry leaf per query at least, the whole tree at most."""
@@ -308,15 +332,12 @@ def work(case):
         return {"bytes": 2 * 12 * ns + 12 * nt + 16 * entries, "flops": ns * (32 * 8 + 40 * k)}
     n, nq = case["n"], case["nq"]
     if kind == "forest":
-        # log-uniform radii over trees of geometric sizes: a mean over both
-        sizes = _split(n, case["trees"], 10_000, 100.0)
-        chords = [1e-4 * 100 ** ((i + 0.5) / 16) for i in range(16)]
-        hits = sum(_hits(m, r) for m in sizes for r in chords) / (len(sizes) * len(chords))
+        hits = _mean_hits(case)
         out = 44 if case["family"] == "best" else 8 + 8 * hits
         scanned = max(32, hits)
         io = 12 + 4 + 4
     elif kind == "within":
-        hits = _hits(n, case["chord"])
+        hits = _mean_hits(case)
         out, scanned, io = 8 + (sa + 4) * hits, max(32, hits), 3 * sa
     elif kind == "one":
         out, scanned, io = sa + 4, 32, d * sa
