@@ -1049,209 +1049,6 @@ __global__ void __launch_bounds__(256) k_periodic_within_fill(
   });
 }
 
-// Segments of at most 32 hits: one warp, bitonic network on (distance, position)
-// so equal distances keep traversal order (a stable sort, as Vec::sort).
-template <typename A>
-__device__ __forceinline__ bool key_less(A da, uint32_t pa, A db, uint32_t pb) {
-  return da < db || (da == db && pa < pb);
-}
-
-// Stable sort of one segment of n <= N hits by its own thread: the segment is
-// loaded into registers (padding +inf after it), insertion-sorted by a fully
-// unrolled network of adjacent compare-swaps that swap only strictly greater
-// keys (so equal keys keep their order and padding stays behind), and written
-// back.
-template <typename A, int N>
-__device__ __forceinline__ void small_segment_sort(A* __restrict__ d, uint32_t* __restrict__ it,
-                                                   uint32_t n) {
-  A kd[N];
-  uint32_t kv[N];
-#pragma unroll
-  for (int j = 0; j < N; ++j) {
-    kd[j] = uint32_t(j) < n ? d[j] : inf_of<A>();
-    kv[j] = uint32_t(j) < n ? it[j] : 0u;
-  }
-#pragma unroll
-  for (int a = 1; a < N; ++a) {
-#pragma unroll
-    for (int j = a; j > 0; --j) {
-      const bool sw = kd[j - 1] > kd[j];
-      const A td = kd[j - 1];
-      const uint32_t tv = kv[j - 1];
-      kd[j - 1] = sw ? kd[j] : td;
-      kv[j - 1] = sw ? kv[j] : tv;
-      kd[j] = sw ? td : kd[j];
-      kv[j] = sw ? tv : kv[j];
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < N; ++j)
-    if (uint32_t(j) < n) {
-      d[j] = kd[j];
-      it[j] = kv[j];
-    }
-}
-
-// Segments of up to 32 hits.  A warp takes 32 segments at a time (lane l
-// reads segment base + l's bounds, coalesced): segments of 2..kThreadSort
-// hits are sorted in registers by their own lane (small_segment_sort), and
-// the warp then bitonic-sorts its segments of
-// kThreadSort+1..32 hits one after another on (key, position).
-template <typename A>
-__global__ void __launch_bounds__(256) k_seg_sort_warp(const uint64_t* __restrict__ offsets,
-                                                       uint64_t nq, uint64_t capacity,
-                                                       A* __restrict__ d,
-                                                       uint32_t* __restrict__ it) {
-  constexpr uint64_t kThreadSort = 8;
-  const int lane = threadIdx.x & 31;
-  const uint64_t warp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
-  for (uint64_t base = warp * 32; base < nq; base += nwarps * 32) {
-    const uint64_t s = base + lane;
-    uint64_t o = 0, n = 0;
-    if (s < nq) {
-      o = min(offsets[s], capacity);
-      n = min(offsets[s + 1], capacity) - o;
-    }
-    if (n >= 2 && n <= 4) {
-      small_segment_sort<A, 4>(d + o, it + o, uint32_t(n));
-    } else if (n > 4 && n <= kThreadSort) {
-      small_segment_sort<A, kThreadSort>(d + o, it + o, uint32_t(n));
-    }
-    for (unsigned big = __ballot_sync(FULL, n > kThreadSort && n <= 32); big; big &= big - 1) {
-      const int src = __ffs(big) - 1;
-      const uint64_t so = __shfl_sync(FULL, (unsigned long long)o, src);
-      const uint32_t sn = uint32_t(__shfl_sync(FULL, (unsigned long long)n, src));
-      A kd = inf_of<A>();
-      uint32_t kp = 0xffffffffu, kv = 0;
-      if (uint32_t(lane) < sn) { kd = d[so + lane]; kv = it[so + lane]; kp = lane; }
-#pragma unroll
-      for (int size = 2; size <= 32; size <<= 1) {
-#pragma unroll
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-          const A od = __shfl_xor_sync(FULL, kd, stride);
-          const uint32_t op = __shfl_xor_sync(FULL, kp, stride);
-          const uint32_t ov = __shfl_xor_sync(FULL, kv, stride);
-          const bool up = ((lane & size) == 0);
-          const bool lower = (lane & stride) == 0;
-          // lower lane keeps the min when ascending
-          const bool other_less = key_less(od, op, kd, kp);
-          const bool take = lower ? (up ? other_less : !other_less) : (up ? !other_less : other_less);
-          if (take && !(od == kd && op == kp)) { kd = od; kp = op; kv = ov; }
-        }
-      }
-      if (uint32_t(lane) < sn) { d[so + lane] = kd; it[so + lane] = kv; }
-    }
-  }
-}
-
-// Stable merge step (merge path): out[lo..hi) from runs a[0..na) and b[0..nb),
-// ties taken from `a` first.
-template <typename A>
-__device__ __forceinline__ void merge_range(const A* ad, const uint32_t* ai, uint32_t na,
-                                            const A* bd, const uint32_t* bi, uint32_t nb,
-                                            A* od, uint32_t* oi, uint32_t lo, uint32_t hi) {
-  if (lo >= hi) return;
-  uint32_t l = lo > nb ? lo - nb : 0, h = lo < na ? lo : na;
-  while (l < h) {
-    const uint32_t mid = (l + h) >> 1;
-    if (!(bd[lo - mid - 1] < ad[mid])) l = mid + 1;  // ad[mid] <= bd[...]: a first
-    else h = mid;
-  }
-  uint32_t x = l, y = lo - l;
-  for (uint32_t o = lo; o < hi; ++o) {
-    bool take_a = x < na && (y >= nb || !(bd[y] < ad[x]));
-    if (take_a) { od[o] = ad[x]; oi[o] = ai[x]; ++x; }
-    else { od[o] = bd[y]; oi[o] = bi[y]; ++y; }
-  }
-}
-
-// Bottom-up stable merge sort of one segment by the whole block, ping-ponging
-// between (d0, i0) and (d1, i1).  Returns true if the result ended in (d1, i1).
-template <typename A>
-__device__ bool block_merge_sort(A* d0, uint32_t* i0, A* d1, uint32_t* i1, uint32_t n) {
-  bool in1 = false;
-  for (uint32_t width = 1; width < n; width <<= 1) {
-    A* sd = in1 ? d1 : d0;
-    uint32_t* si = in1 ? i1 : i0;
-    A* td = in1 ? d0 : d1;
-    uint32_t* ti = in1 ? i0 : i1;
-    const uint32_t per = (n + blockDim.x - 1) / blockDim.x;
-    const uint32_t lo = threadIdx.x * per;
-    const uint32_t hi = min(n, lo + per);
-    // each thread's output range may span several run pairs
-    uint32_t o = lo;
-    while (o < hi) {
-      const uint32_t pair = o / (2 * width);
-      const uint32_t start = pair * 2 * width;
-      const uint32_t mid = min(n, start + width);
-      const uint32_t end = min(n, start + 2 * width);
-      const uint32_t stop = min(hi, end);
-      merge_range<A>(sd + start, si + start, mid - start, sd + mid, si + mid, end - mid,
-                     td + start, ti + start, o - start, stop - start);
-      o = stop;
-    }
-    __syncthreads();
-    in1 = !in1;
-  }
-  return in1;
-}
-
-// Segments longer than 32: one block per group of 256 segments; each long
-// segment is sorted by the whole block in shared memory when it fits, else in
-// global memory with `scratch` as the second buffer.
-template <typename A>
-__global__ void __launch_bounds__(256) k_seg_sort_block(const uint64_t* __restrict__ offsets,
-                                                        uint64_t nq, uint64_t capacity,
-                                                        A* __restrict__ d,
-                                                        uint32_t* __restrict__ it,
-                                                        A* __restrict__ scratch_d,
-                                                        uint32_t* __restrict__ scratch_i,
-                                                        uint32_t smem_cap) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ uint32_t list[256];
-  __shared__ uint32_t list_n;
-  const uint64_t first = uint64_t(blockIdx.x) * 256;
-  if (threadIdx.x == 0) list_n = 0;
-  __syncthreads();
-  {
-    const uint64_t s = first + threadIdx.x;
-    if (s < nq) {
-      const uint64_t n = min(offsets[s + 1], capacity) - min(offsets[s], capacity);
-      if (n > 32) list[atomicAdd(&list_n, 1u)] = uint32_t(threadIdx.x);
-    }
-  }
-  __syncthreads();
-  const uint32_t cnt = list_n;
-  A* sd0 = reinterpret_cast<A*>(smem_raw);
-  A* sd1 = sd0 + smem_cap;
-  uint32_t* si0 = reinterpret_cast<uint32_t*>(sd1 + smem_cap);
-  uint32_t* si1 = si0 + smem_cap;
-  for (uint32_t j = 0; j < cnt; ++j) {
-    const uint64_t s = first + list[j];
-    const uint64_t o = min(offsets[s], capacity);
-    const uint32_t n = uint32_t(min(offsets[s + 1], capacity) - o);
-    if (n <= smem_cap) {
-      for (uint32_t x = threadIdx.x; x < n; x += blockDim.x) { sd0[x] = d[o + x]; si0[x] = it[o + x]; }
-      __syncthreads();
-      const bool in1 = block_merge_sort<A>(sd0, si0, sd1, si1, n);
-      const A* rd = in1 ? sd1 : sd0;
-      const uint32_t* ri = in1 ? si1 : si0;
-      for (uint32_t x = threadIdx.x; x < n; x += blockDim.x) { d[o + x] = rd[x]; it[o + x] = ri[x]; }
-      __syncthreads();
-    } else {
-      const bool in1 = block_merge_sort<A>(d + o, it + o, scratch_d + o, scratch_i + o, n);
-      if (in1) {
-        for (uint32_t x = threadIdx.x; x < n; x += blockDim.x) {
-          d[o + x] = scratch_d[o + x];
-          it[o + x] = scratch_i[o + x];
-        }
-      }
-      __syncthreads();
-    }
-  }
-}
-
 }  // namespace kgpu
 
 namespace kgpu {

@@ -440,30 +440,6 @@ cudaError_t launch_within_fill(const DeviceTree& t, const QueryLaunch& q,
 }
 
 template <typename A>
-cudaError_t launch_seg_sort(const uint64_t* offsets, uint64_t nq, uint64_t capacity, A* d,
-                            uint32_t* it, A* scratch_d, uint32_t* scratch_i, cudaStream_t s) {
-  if (nq == 0) return cudaSuccess;
-  {
-    auto kern = k_seg_sort_warp<A>;
-    const int grid = grid_for(kern, 0, (nq + 31) / 32);
-    kern<<<grid, 256, 0, s>>>(offsets, nq, capacity, d, it);
-    g_launches++;
-  }
-  {
-    // shared-memory ping-pong buffers for segments up to `cap` hits
-    const uint32_t cap = 4096;
-    const size_t smem = size_t(cap) * 2 * (sizeof(A) + sizeof(uint32_t));
-    auto kern = k_seg_sort_block<A>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    const uint64_t blocks = (nq + 255) / 256;
-    kern<<<unsigned(blocks), 256, smem, s>>>(offsets, nq, capacity, d, it, scratch_d, scratch_i,
-                                             cap);
-    g_launches++;
-  }
-  return cudaGetLastError();
-}
-
-template <typename A>
 cudaError_t launch_spatial_order(const DeviceTree& t, const QueryLaunch& q, uint32_t* order,
                                  void* scratch) {
   const TreeView<A> tv = make_view<A>(t);
@@ -533,8 +509,6 @@ cudaError_t launch_spatial_order(const DeviceTree& t, const QueryLaunch& q, uint
   template cudaError_t launch_within_count<A>(const DeviceTree&, const QueryLaunch&, uint64_t*); \
   template cudaError_t launch_within_fill<A>(const DeviceTree&, const QueryLaunch&,              \
                                              const uint64_t*);                                   \
-  template cudaError_t launch_seg_sort<A>(const uint64_t*, uint64_t, uint64_t, A*, uint32_t*,    \
-                                          A*, uint32_t*, cudaStream_t);                          \
   template cudaError_t launch_spatial_order<A>(const DeviceTree&, const QueryLaunch&, uint32_t*, \
                                                void*);                                           \
   }
