@@ -857,6 +857,8 @@ cudaError_t maybe_spatial_order(const DeviceTree& dt, const kgpu_query_desc* d, 
 
 template <typename A>
 cudaError_t run_fixed(const DeviceTree& dt, QueryLaunch& q) {
+  // statistics count the asked-for engine's walk
+  if (!q.stats) q.engine = engine_for(dt, q);
   bool handled = false;
   const cudaError_t e = periodic_fast<A>(dt, q, handled);
   return handled ? e : launch_fixed<A>(dt, q);
@@ -1091,6 +1093,7 @@ int32_t kgpu_query_radius_count(kgpu_tree* t, const kgpu_query_desc* d, const vo
   apply_periodic(dt, d, q);
   q.engine = engine_of(d->flags);
   apply_tuning(d->tuning, q);
+  q.engine = engine_for(dt, q);
   q.stream = s;
   uint64_t* doff = offsets;
   if (host) {
@@ -1160,6 +1163,7 @@ int32_t kgpu_query_radius_fill(kgpu_tree* t, const kgpu_query_desc* d, const voi
   apply_periodic(dt, d, q);
   q.engine = engine_of(d->flags);
   apply_tuning(d->tuning, q);
+  q.engine = engine_for(dt, q);
   q.stream = s;
   const uint64_t* doff = offsets;
   if (host) {

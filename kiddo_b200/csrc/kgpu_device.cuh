@@ -578,6 +578,7 @@ __device__ __forceinline__ uint32_t scan_nearest_one(const TreeView<A>& tv, uint
       A c[K];
       load_point<A, K>(base, len, p, c, it);
       dd = point_dist<M, A, K>(c, q);
+      if (dd != dd) dd = INF;  // a NaN distance never wins, and must not split the warp's minimum
     }
     A m = dd;
 #pragma unroll

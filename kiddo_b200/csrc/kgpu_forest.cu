@@ -98,6 +98,7 @@ int forest_launch(kgpu_forest* f, const kgpu_query_desc* d, const void* queries,
   apply_periodic(f->meta, d, q);
   q.engine = engine_of(d->flags);
   apply_tuning(d->tuning, q);
+  q.engine = engine_for(f->meta, q);
   return KGPU_OK;
 }
 

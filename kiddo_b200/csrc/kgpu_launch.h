@@ -101,6 +101,49 @@ inline void apply_tuning(uint32_t tuning, QueryLaunch& q) {
   if (chunk_log2 >= 5 && chunk_log2 <= 10) q.chunk = 1u << chunk_log2;
 }
 
+// The engine of a batch that asks for none: small batches of 2-D and 3-D trees
+// take the warp engine.  A thread walks its query alone, so a batch too small
+// to fill the GPU with threads takes as long as one thread's walk (0.1 to 1
+// ms); a warp answers a query in about a twentieth of that, and the engines
+// meet where the warps' throughput limit reaches the thread's latency.
+// Measured, 1M-point uniform and clustered trees and 10k points (thread / warp
+// engine, us, both sides of the line): nearest_one f32 32768 queries 129 / 84,
+// 65535 145 / 146; nearest_n f32 k = 8 65535 305 / 286, 98304 331 / 436; k = 16
+// 65535 468 / 371, 98304 505 / 556; k = 32 98304 1064 / 781, 131072 1093 / 1024,
+// 262144 1824 / 2012; best_n 65535 308 / 234, 98304 341 / 348; within 49152 560
+// / 451, 65536 541 / 587; periodic within f64 32768 1049 / 904, 49152 1069 /
+// 1217.  Periodic lists (65535 queries: f32 k = 8 836 / 591, f64 k = 16 1445 /
+// 1190) end where the plain-walk path begins (kgpu_periodic_fast.cu).  f64 lists above 32 entries are the warp engine's at every size
+// (393216 queries: k = 40 9319 / 8491, k = 64 18620 / 12521): the per-thread
+// lists leave two blocks per SM.  Explicit engines, Donnelly and Mapped trees
+// (thread walks only) and lists kept in output rows are not touched.
+inline int engine_for(const DeviceTree& t, const QueryLaunch& q) {
+  if (q.engine != 0 || t.scalar_walk() || (t.dims != 2 && t.dims != 3)) return q.engine;
+  const uint64_t k = uint64_t(q.k > 0 ? q.k : 1);
+  uint64_t below = 0;
+  switch (q.family) {
+    case KGPU_NEAREST_ONE:
+      below = 40960;
+      break;
+    case KGPU_NEAREST_N:
+    case KGPU_NEAREST_N_WITHIN:
+      if (q.periodic) below = k <= 32 ? 65536 : 0;
+      else if (k <= 32) below = 40960 + 2560 * k;
+      else below = t.dtype == KGPU_F64 ? ~uint64_t(0) : 65536;
+      break;
+    case KGPU_BEST_N_WITHIN:
+      below = 81920;
+      break;
+    case KGPU_WITHIN:
+    case KGPU_WITHIN_UNSORTED:
+      below = q.periodic ? 40960 : 57344;
+      break;
+    default:  // approx: one leaf per query, the thread engine's at every size
+      break;
+  }
+  return q.nq < below ? 1 : q.engine;
+}
+
 // Fixed-size families: dispatches to the thread engine (2-D/3-D trees) or the
 // warp engine (everything else, periodic included).
 template <typename A> cudaError_t launch_fixed(const DeviceTree& t, const QueryLaunch& q);

@@ -108,6 +108,7 @@ extern "C" int32_t kgpu_query_radius_count_noalloc(kgpu_tree* t, const kgpu_quer
   apply_periodic(dt, d, q);
   q.engine = engine_of(d->flags);
   apply_tuning(d->tuning, q);
+  q.engine = engine_for(t->dt, q);
   q.queries = queries;
   q.stream = s;
   if (nq) {
