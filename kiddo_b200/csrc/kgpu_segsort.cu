@@ -28,6 +28,7 @@
 
 #include <cuda_runtime.h>
 
+#include "kgpu_bitonic.cuh"
 #include "kgpu_devbuf.h"
 #include "kgpu_device.cuh"
 #include "kgpu_launch.h"
@@ -70,10 +71,9 @@ struct KeyF64 {
 template <typename A>
 using KeyOf = typename std::conditional<sizeof(A) == 4, KeyF32, KeyF64>::type;
 
-// N keys in shared memory, one pad slot after every 16, so that threads 8, 16
-// or 32 entries apart touch different banks.
-template <typename Key>
-struct KeyStore;
+}  // namespace
+
+// in shared memory, one pad slot after every 16
 template <>
 struct KeyStore<KeyF32> {
   unsigned long long* v;
@@ -104,109 +104,7 @@ struct KeyStore<KeyF64> {
   }
 };
 
-// ---- networks -----------------------------------------------------------------
-// All comparators ascend (the lower index keeps the smaller key): the first
-// step of each power of two pairs index i with its mirror in the block, the
-// later steps pair i with i ^ stride.
-template <typename Key>
-__device__ __forceinline__ void order_pair(Key& a, Key& b) {
-  const bool sw = b < a;
-  const Key t = a;
-  a = sw ? b : a;
-  b = sw ? t : b;
-}
-
-// Strides STRIDE, STRIDE / 2, ... 1 over a warp's 32 * E keys held blocked
-// (lane t has indices t * E + e).
-template <typename Key, int E, int STRIDE>
-__device__ __forceinline__ void warp_strides(Key (&k)[E], int lane) {
-  if constexpr (STRIDE >= E) {
-    constexpr int M = STRIDE / E;
-    const bool low = (lane & M) == 0;
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const Key o = k[e].from_lane(M);
-      k[e] = ((o < k[e]) == low) ? o : k[e];
-    }
-    if constexpr (STRIDE > 1) warp_strides<Key, E, STRIDE / 2>(k, lane);
-  } else if constexpr (STRIDE >= 1) {
-#pragma unroll
-    for (int e = 0; e < E; ++e)
-      if ((e & STRIDE) == 0) order_pair(k[e], k[e + STRIDE]);
-    if constexpr (STRIDE > 1) warp_strides<Key, E, STRIDE / 2>(k, lane);
-  }
-}
-
-// Sorts the warp's 32 * E keys: sizes SIZE, 2 SIZE, ... 32 E.
-template <typename Key, int E, int SIZE = 2>
-__device__ __forceinline__ void warp_sort(Key (&k)[E], int lane) {
-  if constexpr (SIZE <= 32 * E) {
-    if constexpr (SIZE <= E) {
-#pragma unroll
-      for (int e = 0; e < E; ++e)
-        if ((e & (SIZE / 2)) == 0) order_pair(k[e], k[e ^ (SIZE - 1)]);
-    } else {
-      constexpr int M = SIZE / E - 1;
-      const bool low = (lane & (SIZE / E / 2)) == 0;
-      if constexpr (E == 1) {
-        const Key o = k[0].from_lane(M);
-        k[0] = ((o < k[0]) == low) ? o : k[0];
-      } else {
-#pragma unroll
-        for (int e = 0; e < E / 2; ++e) {
-          const Key a = k[E - 1 - e].from_lane(M), b = k[e].from_lane(M);
-          k[e] = ((a < k[e]) == low) ? a : k[e];
-          k[E - 1 - e] = ((b < k[E - 1 - e]) == low) ? b : k[E - 1 - e];
-        }
-      }
-    }
-    if constexpr (SIZE > 2) warp_strides<Key, E, SIZE / 4>(k, lane);
-    warp_sort<Key, E, SIZE * 2>(k, lane);
-  }
-}
-
-// In-thread strides of keys held strided (thread t has indices e * T + t):
-// index strides ES * T, ... T.
-template <typename Key, int E, int ES>
-__device__ __forceinline__ void thread_strides(Key (&k)[E]) {
-  if constexpr (ES >= 1) {
-#pragma unroll
-    for (int e = 0; e < E; ++e)
-      if ((e & ES) == 0) order_pair(k[e], k[e + ES]);
-    thread_strides<Key, E, ES / 2>(k);
-  }
-}
-
-// Sizes SIZE, 2 SIZE, ... T * E of a block of T threads whose warps hold
-// sorted runs of SIZE / 2 keys, blocked in and blocked out.  Between warps the
-// keys go through shared memory: written with the upper half of every
-// SIZE-block mirrored (which turns the mirrored first step into a plain
-// stride), read strided for the strides from SIZE / 2 down to T, and written
-// back for the strides inside a warp.  Needs 32 * E >= T.
-template <typename Key, int T, int E, int SIZE>
-__device__ __forceinline__ void block_merges(Key (&k)[E], KeyStore<Key>& sm, int tid) {
-  static_assert(32 * E >= T, "a warp's run must reach the strided strides");
-  if constexpr (SIZE <= T * E) {
-    __syncthreads();
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const uint32_t i = uint32_t(tid) * E + e;
-      sm.put((i & (SIZE / 2)) ? i ^ (SIZE / 2 - 1) : i, k[e]);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int e = 0; e < E; ++e) k[e] = sm.get(uint32_t(e) * T + tid);
-    thread_strides<Key, E, SIZE / 2 / T>(k);
-    // each thread rewrites the slots that it read
-#pragma unroll
-    for (int e = 0; e < E; ++e) sm.put(uint32_t(e) * T + tid, k[e]);
-    __syncthreads();
-#pragma unroll
-    for (int e = 0; e < E; ++e) k[e] = sm.get(uint32_t(tid) * E + e);
-    warp_strides<Key, E, (T / 2 < 16 * E ? T / 2 : 16 * E)>(k, tid & 31);
-    block_merges<Key, T, E, SIZE * 2>(k, sm, tid);
-  }
-}
+namespace {
 
 // Stable sort of the n <= T * E entries at (d, it) by T threads (a warp of its
 // own slice of shared memory when T == 32, else the whole block).
