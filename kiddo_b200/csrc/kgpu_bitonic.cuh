@@ -5,8 +5,11 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 
 #include <cuda_runtime.h>
+
+#include "kgpu_device.cuh"
 
 namespace kgpu {
 
@@ -14,6 +17,74 @@ namespace kgpu {
 // or 32 entries apart touch different banks.
 template <typename Key>
 struct KeyStore;
+
+// Distances with a place: unique keys, so any sort of them is a stable sort of
+// the distances.  Distances are +0 or more and never NaN, so their bit patterns
+// order like their values.
+// f32: distance bits above the position in one 64-bit word.  f64: the distance
+// bits and the position.
+struct KeyF32 {
+  unsigned long long v;
+  __device__ __forceinline__ static KeyF32 make(float d, uint32_t p) {
+    return {(static_cast<unsigned long long>(__float_as_uint(d)) << 32) | p};
+  }
+  __device__ __forceinline__ static KeyF32 last() { return {~0ull}; }
+  __device__ __forceinline__ bool operator<(const KeyF32& o) const { return v < o.v; }
+  __device__ __forceinline__ float dist() const { return __uint_as_float(uint32_t(v >> 32)); }
+  __device__ __forceinline__ uint32_t pos() const { return uint32_t(v); }
+  __device__ __forceinline__ KeyF32 from_lane(int mask) const {
+    return {__shfl_xor_sync(FULL, v, mask)};
+  }
+};
+struct KeyF64 {
+  unsigned long long v;
+  uint32_t p;
+  __device__ __forceinline__ static KeyF64 make(double d, uint32_t p) {
+    return {static_cast<unsigned long long>(__double_as_longlong(d)), p};
+  }
+  __device__ __forceinline__ static KeyF64 last() { return {~0ull, ~0u}; }
+  __device__ __forceinline__ bool operator<(const KeyF64& o) const {
+    return v < o.v || (v == o.v && p < o.p);
+  }
+  __device__ __forceinline__ double dist() const { return __longlong_as_double((long long)v); }
+  __device__ __forceinline__ uint32_t pos() const { return p; }
+  __device__ __forceinline__ KeyF64 from_lane(int mask) const {
+    return {__shfl_xor_sync(FULL, v, mask), __shfl_xor_sync(FULL, p, mask)};
+  }
+};
+template <typename A>
+using KeyOf = typename std::conditional<sizeof(A) == 4, KeyF32, KeyF64>::type;
+
+// in shared memory, one pad slot after every 16
+template <>
+struct KeyStore<KeyF32> {
+  unsigned long long* v;
+  __host__ __device__ static constexpr size_t slots(uint32_t n) { return n + n / 16; }
+  __host__ __device__ static constexpr size_t bytes(uint32_t n) { return slots(n) * 8; }
+  __device__ static KeyStore at(unsigned char* p, uint32_t) {
+    return {reinterpret_cast<unsigned long long*>(p)};
+  }
+  __device__ __forceinline__ KeyF32 get(uint32_t i) const { return {v[i + (i >> 4)]}; }
+  __device__ __forceinline__ void put(uint32_t i, const KeyF32& k) { v[i + (i >> 4)] = k.v; }
+};
+template <>
+struct KeyStore<KeyF64> {
+  unsigned long long* v;
+  uint32_t* p;
+  __host__ __device__ static constexpr size_t slots(uint32_t n) { return n + n / 16; }
+  __host__ __device__ static constexpr size_t bytes(uint32_t n) { return slots(n) * 12; }
+  __device__ static KeyStore at(unsigned char* m, uint32_t n) {
+    unsigned long long* v = reinterpret_cast<unsigned long long*>(m);
+    return {v, reinterpret_cast<uint32_t*>(v + slots(n))};
+  }
+  __device__ __forceinline__ KeyF64 get(uint32_t i) const {
+    return {v[i + (i >> 4)], p[i + (i >> 4)]};
+  }
+  __device__ __forceinline__ void put(uint32_t i, const KeyF64& k) {
+    v[i + (i >> 4)] = k.v;
+    p[i + (i >> 4)] = k.p;
+  }
+};
 
 // All comparators ascend (the lower index keeps the smaller key): the first
 // step of each power of two pairs index i with its mirror in the block, the

@@ -259,12 +259,15 @@ cudaError_t launch_tfixed_stems(const DeviceTree& t, const QueryLaunch& q) {
             case KGPU_NEAREST_N:
             case KGPU_NEAREST_N_WITHIN:
               // warp-cooperative leaf scans with lists in the output rows: on
-              // request, and by default for f64 lists above 20 entries, where
-              // per-thread lists in shared memory cut the blocks per SM (16M
-              // queries, f64, k = 24: 95 against 101 ms; k = 32: 115 against
-              // 261 ms; f32 up to k = 32 and f64 up to 16 stay per thread)
-              if ((q.engine == 3 || (q.engine == 0 && sizeof(A) == 8 && q.k > 20)) && q.sorted &&
-                  q.k <= kMaxK) {
+              // request, and by default for longer lists, where the
+              // per-thread insertions cost more and the per-thread lists in
+              // shared memory cut the blocks per SM.  4M queries of a
+              // clustered 4M-point tree (thread / cooperative, ms): f32 3-D
+              // k = 16 8.07 / 9.75, 20 11.32 / 11.44, 24 13.83 / 12.27, 32
+              // 25.81 / 14.43; f32 2-D 16 4.51 / 5.37, 24 7.73 / 6.69; f64 3-D
+              // 12 9.75 / 11.68, 16 16.33 / 13.70, 32 65.63 / 21.28
+              if ((q.engine == 3 || (q.engine == 0 && q.k > (sizeof(A) == 8 ? 13 : 20))) &&
+                  q.sorted && q.k <= kMaxK) {
                 const size_t csmem = size_t(levels) * 256 * (STEMS ? 2 * sizeof(A) + 4 : sizeof(A));
                 auto kern = k_tnn_coop<A, K, M, EX, STEMS>;
                 cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
