@@ -810,6 +810,12 @@ cudaError_t with_work_counter(const QueryLaunch& q, F&& launch) {
   return launch(qw);
 }
 
+// The same for the radius passes, whose warp engine keeps its fixed shares.
+template <typename F>
+cudaError_t with_walk_counter(const QueryLaunch& q, F&& launch) {
+  return q.engine == 1 ? launch(q) : with_work_counter(q, launch);
+}
+
 template <typename A>
 cudaError_t launch_fixed(const DeviceTree& t, const QueryLaunch& q) {
   // thread engine for 2-D/3-D trees; periodic nearest_one stays on the warp
@@ -1114,8 +1120,10 @@ int32_t kgpu_query_radius_count(kgpu_tree* t, const kgpu_query_desc* d, const vo
   if ((e = maybe_spatial_order(dt, d, q, bord, bos, s)) != cudaSuccess)
     return cuda_fail(e, "ordering the batch");
   if (nq) {
-    e = dt.dtype == KGPU_F64 ? launch_within_count<double>(dt, q, doff)
-                             : launch_within_count<float>(dt, q, doff);
+    e = with_walk_counter(q, [&](const QueryLaunch& qw) {
+      return dt.dtype == KGPU_F64 ? launch_within_count<double>(dt, qw, doff)
+                                  : launch_within_count<float>(dt, qw, doff);
+    });
     if (e != cudaSuccess) return cuda_fail(e, "launching the counting kernel");
   }
   e = launch_exclusive_scan(doff, doff, nq, btmp.p, s);
@@ -1186,8 +1194,10 @@ int32_t kgpu_query_radius_fill(kgpu_tree* t, const kgpu_query_desc* d, const voi
   DevBuf bord, bos;
   if ((e = maybe_spatial_order(dt, d, q, bord, bos, s)) != cudaSuccess)
     return cuda_fail(e, "ordering the batch");
-  e = dt.dtype == KGPU_F64 ? launch_within_fill<double>(dt, q, doff)
-                           : launch_within_fill<float>(dt, q, doff);
+  e = with_walk_counter(q, [&](const QueryLaunch& qw) {
+    return dt.dtype == KGPU_F64 ? launch_within_fill<double>(dt, qw, doff)
+                                : launch_within_fill<float>(dt, qw, doff);
+  });
   if (e != cudaSuccess) return cuda_fail(e, "launching the fill kernel");
   if (sorted) {
     if ((e = sd.alloc(total * sa, s)) != cudaSuccess || (e = si.alloc(total * 4, s)) != cudaSuccess)

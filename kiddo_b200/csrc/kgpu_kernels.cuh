@@ -255,7 +255,7 @@ __device__ __forceinline__ void flush_stats(unsigned long long* stats, const Tra
 }
 
 // Queries handed out to the lanes of one warp in chunks of Batch::chunk
-// queries (64 unless tuned): from the batch's work counter when it has one,
+// queries (32 unless tuned): from the batch's work counter when it has one,
 // else chunks gw, gw + W, gw + 2W, ... (gw = this warp, W = warps in the
 // grid).  Interleaving spreads the costly regions of a leaf-ordered batch
 // evenly over the warps.
@@ -295,8 +295,8 @@ struct LaneFeeder {
   }
 };
 
-// Warp-uniform: once at least Batch::refill lanes of the warp (24 unless
-// tuned), or all of them, have no query, gives each of them the next query of
+// Warp-uniform: once at least Batch::refill lanes of the warp (8 to 24 by kernel
+// unless tuned), or all of them, have no query, gives each of them the next query of
 // the batch (lowest lanes first, so new queries start side by side); returns
 // whether any lane of the warp still has a query.
 template <typename A>

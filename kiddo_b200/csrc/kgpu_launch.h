@@ -63,8 +63,8 @@ struct QueryLaunch {
   uint32_t* out_i = nullptr;
   uint32_t* out_c = nullptr;
   unsigned long long* stats = nullptr;  // optional [stems, leaves, points] totals
-  uint32_t chunk = 64;            // queries handed to a warp at a time (lane-refilled drivers)
-  int refill = 24;                // idle lanes a warp waits for before refilling them
+  uint32_t chunk = 0;             // queries handed to a warp at a time (lane-refilled drivers)
+  int refill = 0;                 // idle lanes a warp waits for before refilling them; 0: defaults
   int engine = 0;                 // 0 auto, 1 warp per query, 2 thread per query,
                                   // 3 thread walks with warp-cooperative leaf scans
   bool periodic = false;          // periodic boundary conditions
@@ -93,7 +93,7 @@ inline int engine_of(uint32_t flags) {
 }
 
 // The launch knobs of kgpu_query_desc::tuning (KGPU_TUNE_*); 0 fields keep
-// the defaults (24 idle lanes, 64-query chunks).
+// the defaults (make_batch).
 inline void apply_tuning(uint32_t tuning, QueryLaunch& q) {
   const uint32_t refill = tuning & 0x3fu;
   const uint32_t chunk_log2 = (tuning >> 8) & 0xfu;

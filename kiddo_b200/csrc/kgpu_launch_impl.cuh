@@ -66,8 +66,18 @@ inline cudaError_t with_excl(bool e, F&& f) {
   return f(std::false_type());
 }
 
+// `refill`: idle lanes the kernel's warps wait for, unless the query tunes it.
+// Per-thread leaf scans (nearest_n) want a warp's queries in step and wait for
+// 24 (kNN16, 16M queries: 30.9 ms, 16 idle lanes 32.9, 8 36.8); nearest_one,
+// whose scans are short, 16 (1M f64 queries: 450 us at 24, 425 at 16); kernels
+// that scan a leaf with the whole warp only idle in the walk, and refill at 8
+// (best_n over 32 catalogues, 4M queries: 7.47 ms at 24, 7.11 at 16, 7.03 at 8).
+// Chunks of 32 against 64 shorten the end of a launch, where warps wait for the
+// last chunks: best_n 8.09 to 7.47 ms, kNN8 over 16 clouds 1.95 to 1.89 ms; kNN16
+// over 16M queries, whose end is a small part, keeps 64 (30.43 ms, 30.55 at 32).
+constexpr int kRefillScan = 24, kRefillOne = 16, kRefillCoop = 8;
 template <typename A>
-inline Batch<A> make_batch(const QueryLaunch& q) {
+inline Batch<A> make_batch(const QueryLaunch& q, int refill = kRefillScan) {
   Batch<A> b;
   b.Q = static_cast<const A*>(q.queries);
   b.order = q.order;
@@ -77,8 +87,8 @@ inline Batch<A> make_batch(const QueryLaunch& q) {
   b.n_trees = q.n_trees;
   b.radii = static_cast<const A*>(q.radii);
   b.work = q.work;
-  b.chunk = q.chunk;
-  b.refill = q.refill;
+  b.chunk = q.chunk ? q.chunk : refill == kRefillScan && q.nq >= (uint64_t(1) << 23) ? 64 : 32;
+  b.refill = q.refill ? q.refill : refill;
   b.nq_dev = q.nq_dev;
   return b;
 }
@@ -191,7 +201,10 @@ cudaError_t launch_wfixed(const DeviceTree& t, const QueryLaunch& q) {
 template <typename A, int STEMS>
 cudaError_t launch_tfixed_stems(const DeviceTree& t, const QueryLaunch& q) {
   const TreeView<A> tv = make_view<A>(t);
-  const Batch<A> b = make_batch<A>(q);
+  const Batch<A> b = make_batch<A>(
+      q, q.family == KGPU_NEAREST_ONE ? kRefillOne
+                                      : q.family == KGPU_BEST_N_WITHIN ? kRefillCoop : kRefillScan);
+  const Batch<A> coop = make_batch<A>(q, kRefillCoop);
   const A radius = A(q.radius);
   const int levels = t.max_stem_level + 2;
   const bool list = q.family == KGPU_NEAREST_N || q.family == KGPU_NEAREST_N_WITHIN ||
@@ -236,7 +249,7 @@ cudaError_t launch_tfixed_stems(const DeviceTree& t, const QueryLaunch& q) {
             auto kern = k_tperiodic_nn<A, K, M, EX, STEMS>;
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(psmem));
             const int grid = grid_for(kern, psmem, (q.nq + 31) / 32);
-            kern<<<grid, 256, psmem, q.stream>>>(tv, b, box, q.k, radius,
+            kern<<<grid, 256, psmem, q.stream>>>(tv, coop, box, q.k, radius,
                                                   static_cast<A*>(q.out_d), q.out_i, q.out_c,
                                                   q.stats);
             g_launches++;
@@ -273,7 +286,7 @@ cudaError_t launch_tfixed_stems(const DeviceTree& t, const QueryLaunch& q) {
                 cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      int(csmem));
                 const int grid = grid_for(kern, csmem, (q.nq + 31) / 32);
-                kern<<<grid, 256, csmem, q.stream>>>(tv, b, levels, q.k, radius,
+                kern<<<grid, 256, csmem, q.stream>>>(tv, coop, levels, q.k, radius,
                                                      static_cast<A*>(q.out_d), q.out_i, q.out_c,
                                                      q.stats);
                 g_launches++;
@@ -302,7 +315,7 @@ cudaError_t launch_tfixed(const DeviceTree& t, const QueryLaunch& q) {
 template <typename A>
 cudaError_t launch_trow(const DeviceTree& t, const QueryLaunch& q) {
   const TreeView<A> tv = make_view<A>(t);
-  const Batch<A> b = make_batch<A>(q);
+  const Batch<A> b = make_batch<A>(q, kRefillCoop);
   const A radius = A(q.radius);
   const int levels = t.max_stem_level + 2;
   const bool best = q.family == KGPU_BEST_N_WITHIN;
@@ -362,7 +375,7 @@ template <typename A, int STEMS>
 cudaError_t launch_within_pass_stems(const DeviceTree& t, const QueryLaunch& q, uint64_t* counts,
                                      const uint64_t* offsets) {
   const TreeView<A> tv = make_view<A>(t);
-  const Batch<A> b = make_batch<A>(q);
+  const Batch<A> b = make_batch<A>(q, kRefillCoop);
   const A radius = A(q.radius);
   return with_dims(t.dims, [&](auto kk) {
     constexpr int K = decltype(kk)::value;
@@ -446,7 +459,7 @@ template <typename A>
 cudaError_t launch_spatial_order(const DeviceTree& t, const QueryLaunch& q, uint32_t* order,
                                  void* scratch) {
   const TreeView<A> tv = make_view<A>(t);
-  const Batch<A> b = make_batch<A>(q);
+  const Batch<A> b = make_batch<A>(q, kRefillCoop);
   const uint64_t nq = q.nq;
   const uint64_t nl = q.forest ? q.total_leaves : (t.leaf_count > 0 ? t.leaf_count : 1);
   // scratch layout: leaf_of[nq] u32 | counts[nl + 1] u64 | scan tiles
