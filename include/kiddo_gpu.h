@@ -369,6 +369,25 @@ int32_t kgpu_query_radius_fill(kgpu_tree* tree, const kgpu_query_desc* desc,
                                const void* queries, uint64_t nq, const uint64_t* offsets,
                                void* out_dists, uint32_t* out_items, void* stream);
 
+/* The same in one walk of the trees: the counting call keeps where the hits are
+ * (a handle of the library's scratch memory, on `stream`), and the filling call
+ * writes them from that.  Device pointers only; neither call can be captured.
+ * kgpu_query_radius_count_keep waits for the total and returns it in *total
+ * (offsets[nq] holds it too).  kgpu_query_radius_fill_kept takes the same
+ * description, queries, offsets and stream, and `total` entries of output; it
+ * may be called again.  kgpu_hits_free releases the handle after the work queued on
+ * `stream`.  A batch whose hits do not fit the handle's scratch is walked
+ * again by the filling call. */
+typedef struct kgpu_hits kgpu_hits;
+int32_t kgpu_query_radius_count_keep(kgpu_tree* tree, const kgpu_query_desc* desc,
+                                     const void* queries, uint64_t nq, uint64_t* offsets,
+                                     uint64_t* total, kgpu_hits** hits, void* stream);
+int32_t kgpu_query_radius_fill_kept(kgpu_tree* tree, const kgpu_query_desc* desc,
+                                    const void* queries, uint64_t nq, const uint64_t* offsets,
+                                    const kgpu_hits* hits, void* out_dists, uint32_t* out_items,
+                                    void* stream);
+int32_t kgpu_hits_free(kgpu_hits* hits);
+
 /* ---- radius count without allocation -------------------------------------
  * No counterpart in the reference: an addition of this engine for callers that
  * cannot allocate device memory while they query (a process whose HBM is
@@ -431,6 +450,16 @@ int32_t kgpu_forest_query_radius_fill(kgpu_forest* forest, const kgpu_query_desc
                                       const void* radii, uint64_t nq, const uint64_t* offsets,
                                       uint64_t capacity, void* out_dists, uint32_t* out_items,
                                       int32_t* status, void* stream);
+/* The forest forms of kgpu_query_radius_count_keep / _fill_kept. */
+int32_t kgpu_forest_query_radius_count_keep(kgpu_forest* forest, const kgpu_query_desc* desc,
+                                            const void* queries, const uint32_t* tree_of,
+                                            const void* radii, uint64_t nq, uint64_t* offsets,
+                                            uint64_t* total, kgpu_hits** hits, void* stream);
+int32_t kgpu_forest_query_radius_fill_kept(kgpu_forest* forest, const kgpu_query_desc* desc,
+                                           const void* queries, const uint32_t* tree_of,
+                                           const void* radii, uint64_t nq, const uint64_t* offsets,
+                                           const kgpu_hits* hits, void* out_dists,
+                                           uint32_t* out_items, void* stream);
 
 /* ---- Chamfer / ICP neighbour loss and its adjoint ------------------------
  * No counterpart in the reference (an addition built on the nearest_n path).

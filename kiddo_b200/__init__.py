@@ -1051,17 +1051,22 @@ class QueryBuilder:
         dev = q.device
         if self.family in (C.WITHIN, C.WITHIN_UNSORTED):
             off = torch.empty(nq + 1, dtype=torch.int64, device=dev)
-            C.check(L.kgpu_query_radius_count(self.tree._h, ctypes.byref(d),
-                                              ctypes.c_void_p(q.data_ptr()), nq,
-                                              ctypes.c_void_p(off.data_ptr()), st))
-            total = int(off[-1].item())
-            dist = torch.empty(max(total, 1), dtype=tdt, device=dev)
-            items = torch.empty(max(total, 1), dtype=torch.int32, device=dev)
-            C.check(L.kgpu_query_radius_fill(self.tree._h, ctypes.byref(d),
-                                             ctypes.c_void_p(q.data_ptr()), nq,
-                                             ctypes.c_void_p(off.data_ptr()),
-                                             ctypes.c_void_p(dist.data_ptr()),
-                                             ctypes.c_void_p(items.data_ptr()), st))
+            total, hits = ctypes.c_uint64(), ctypes.c_void_p()
+            C.check(L.kgpu_query_radius_count_keep(self.tree._h, ctypes.byref(d),
+                                                   ctypes.c_void_p(q.data_ptr()), nq,
+                                                   ctypes.c_void_p(off.data_ptr()),
+                                                   ctypes.byref(total), ctypes.byref(hits), st))
+            try:
+                total = total.value
+                dist = torch.empty(max(total, 1), dtype=tdt, device=dev)
+                items = torch.empty(max(total, 1), dtype=torch.int32, device=dev)
+                C.check(L.kgpu_query_radius_fill_kept(self.tree._h, ctypes.byref(d),
+                                                      ctypes.c_void_p(q.data_ptr()), nq,
+                                                      ctypes.c_void_p(off.data_ptr()), hits,
+                                                      ctypes.c_void_p(dist.data_ptr()),
+                                                      ctypes.c_void_p(items.data_ptr()), st))
+            finally:
+                L.kgpu_hits_free(hits)
             return WithinResult(off, dist[:total], items[:total])
         w = 1 if self.family in (C.NEAREST_ONE, C.APPROX_NEAREST_ONE) else self.max_qty
         dist = torch.empty((nq, w), dtype=tdt, device=dev)
@@ -1132,20 +1137,19 @@ class ForestQueryBuilder(QueryBuilder):
         dev = q.device
         if self.family in (C.WITHIN, C.WITHIN_UNSORTED):
             off = torch.empty(nq + 1, dtype=torch.int64, device=dev)
-            C.check(L.kgpu_forest_query_radius_count(f._h, ctypes.byref(d), vp(q.data_ptr()),
-                                                     vp(tof.data_ptr()), rp, nq,
-                                                     vp(off.data_ptr()), st))
-            total = int(off[-1].item())
-            dist = torch.empty(max(total, 1), dtype=tdt, device=dev)
-            items = torch.empty(max(total, 1), dtype=torch.int32, device=dev)
-            status = torch.zeros(1, dtype=torch.int32, device=dev)
-            C.check(L.kgpu_forest_query_radius_fill(f._h, ctypes.byref(d), vp(q.data_ptr()),
-                                                    vp(tof.data_ptr()), rp, nq,
-                                                    vp(off.data_ptr()), total,
-                                                    vp(dist.data_ptr()), vp(items.data_ptr()),
-                                                    vp(status.data_ptr()), st))
-            if int(status.item()) != 0:
-                raise KiddoGpuError(int(status.item()), "forest fill overflowed its capacity")
+            total, hits = ctypes.c_uint64(), ctypes.c_void_p()
+            C.check(L.kgpu_forest_query_radius_count_keep(
+                f._h, ctypes.byref(d), vp(q.data_ptr()), vp(tof.data_ptr()), rp, nq,
+                vp(off.data_ptr()), ctypes.byref(total), ctypes.byref(hits), st))
+            try:
+                total = total.value
+                dist = torch.empty(max(total, 1), dtype=tdt, device=dev)
+                items = torch.empty(max(total, 1), dtype=torch.int32, device=dev)
+                C.check(L.kgpu_forest_query_radius_fill_kept(
+                    f._h, ctypes.byref(d), vp(q.data_ptr()), vp(tof.data_ptr()), rp, nq,
+                    vp(off.data_ptr()), hits, vp(dist.data_ptr()), vp(items.data_ptr()), st))
+            finally:
+                L.kgpu_hits_free(hits)
             return WithinResult(off, dist[:total], items[:total])
         w = 1 if self.family in (C.NEAREST_ONE, C.APPROX_NEAREST_ONE) else self.max_qty
         dist = torch.empty((nq, w), dtype=tdt, device=dev)

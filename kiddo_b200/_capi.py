@@ -43,7 +43,9 @@ EXPORTED_SYMBOLS = [
     "kgpu_chamfer_backward", "kgpu_tree_create_flatvec", "kgpu_tree_create_vecofarrays",
     "kgpu_scratch_stats", "kgpu_scratch_trim", "kgpu_archive_inspect",
     "kgpu_tree_create_from_archive", "kgpu_tree_create_mapped",
-    "kgpu_tree_create_vecofarrays_mapped",
+    "kgpu_tree_create_vecofarrays_mapped", "kgpu_query_radius_count_keep",
+    "kgpu_query_radius_fill_kept", "kgpu_hits_free", "kgpu_forest_query_radius_count_keep",
+    "kgpu_forest_query_radius_fill_kept",
 ]
 
 
@@ -174,6 +176,21 @@ def lib():
     L.kgpu_query_radius_count.argtypes = [vp, ctypes.POINTER(QueryDesc), vp, u64, vp, vp]
     L.kgpu_query_radius_fill.restype = i32
     L.kgpu_query_radius_fill.argtypes = [vp, ctypes.POINTER(QueryDesc), vp, u64, vp, vp, vp, vp]
+    L.kgpu_query_radius_count_keep.restype = i32
+    L.kgpu_query_radius_count_keep.argtypes = [vp, ctypes.POINTER(QueryDesc), vp, u64, vp,
+                                               ctypes.POINTER(u64), ctypes.POINTER(vp), vp]
+    L.kgpu_query_radius_fill_kept.restype = i32
+    L.kgpu_query_radius_fill_kept.argtypes = [vp, ctypes.POINTER(QueryDesc), vp, u64, vp, vp, vp,
+                                              vp, vp]
+    L.kgpu_hits_free.restype = i32
+    L.kgpu_hits_free.argtypes = [vp]
+    L.kgpu_forest_query_radius_count_keep.restype = i32
+    L.kgpu_forest_query_radius_count_keep.argtypes = [vp, ctypes.POINTER(QueryDesc), vp, vp, vp,
+                                                      u64, vp, ctypes.POINTER(u64),
+                                                      ctypes.POINTER(vp), vp]
+    L.kgpu_forest_query_radius_fill_kept.restype = i32
+    L.kgpu_forest_query_radius_fill_kept.argtypes = [vp, ctypes.POINTER(QueryDesc), vp, vp, vp,
+                                                     u64, vp, vp, vp, vp, vp]
     L.kgpu_launch_count.restype = u64
     L.kgpu_query_radius_count_noalloc.restype = i32
     L.kgpu_query_radius_count_noalloc.argtypes = [vp, ctypes.POINTER(QueryDesc), vp, u64, vp, vp]

@@ -37,6 +37,8 @@ CU_SOURCES = ["kgpu_api.cu", "kgpu_scan.cu", "kgpu_segsort.cu", "kgpu_noalloc.cu
               "kernels_f64_radius.cu",
               "kernels_f32_rows.cu",
               "kernels_f64_rows.cu",
+              "kernels_f32_hits.cu",
+              "kernels_f64_hits.cu",
               ]
 CXX_SOURCES = ["layout_build.cpp", "archive.cpp"]
 HEADERS = sorted(f for f in os.listdir(CSRC) if f.endswith((".h", ".cuh")))

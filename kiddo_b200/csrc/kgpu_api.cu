@@ -17,6 +17,7 @@
 
 #include "../../include/kiddo_gpu.h"
 #include "kgpu_devbuf.h"
+#include "kgpu_hits.h"
 #include "kgpu_internal.h"
 #include "kgpu_launch.h"
 #include "kgpu_tree_impl.h"
@@ -1037,9 +1038,160 @@ int query_host_pipelined(const DeviceTree& dt, const kgpu_query_desc* d, const Q
 }
 
 }  // namespace
+
+// Records are kept where the leaves are rows walked by ThreadWalk: 3-D
+// arithmetic trees without a periodic box, in batches that the thread engine
+// takes.  Room for 16 records per query and what the warps take in advance, at
+// most 2^26 (1.3 GB); it goes back to the pool with the handle.
+int radius_count_keep(const DeviceTree& dt, QueryLaunch& q, uint64_t* offsets, kgpu_hits& hits) {
+  cudaStream_t s = q.stream;
+  const uint64_t nq = q.nq;
+  hits.nq = nq;
+  cudaError_t e;
+  DevBuf tmp;
+  if ((e = tmp.alloc(scan_tmp_bytes(nq), s)) != cudaSuccess ||
+      (e = hits.counters.alloc(4 * sizeof(unsigned long long), s)) != cudaSuccess)
+    return set_error(KGPU_ENOMEM, "device allocation failed");
+  unsigned long long* c = hits.counters.as<unsigned long long>();  // records, total, work
+  if ((e = cudaMemsetAsync(c, 0, 4 * sizeof(unsigned long long), s)) != cudaSuccess)
+    return cuda_fail(e, "memset");
+  const bool f64 = dt.dtype == KGPU_F64;
+  bool keep = dt.dims == 3 && !dt.scalar_walk() && !q.periodic && q.engine != 1 &&
+              nq < (uint64_t(1) << 32);
+  if (keep) {
+    hits.rec.cap = std::min<uint64_t>(16 * nq, uint64_t(1) << 26) + (uint64_t(1) << 20);
+    hits.rec.count = c;
+    // without room for records the batch is walked twice
+    keep = hits.leaf.alloc(hits.rec.cap * sizeof(uint4), s) == cudaSuccess &&
+           hits.query.alloc(hits.rec.cap * 4, s) == cudaSuccess;
+    if (!keep) cudaGetLastError();
+    hits.rec.leaf = hits.leaf.as<uint4>();
+    hits.rec.query = hits.query.as<uint32_t>();
+  }
+  if (nq) {
+    if (q.engine != 1) q.work = c + 2;
+    if (keep)
+      e = f64 ? launch_within_record<double>(dt, q, offsets, hits.rec)
+              : launch_within_record<float>(dt, q, offsets, hits.rec);
+    else
+      e = f64 ? launch_within_count<double>(dt, q, offsets)
+              : launch_within_count<float>(dt, q, offsets);
+    if (e != cudaSuccess) return cuda_fail(e, "launching the counting kernel");
+  }
+  if ((e = launch_exclusive_scan(offsets, offsets, nq, tmp.p, s)) != cudaSuccess)
+    return cuda_fail(e, "launching the scan");
+  unsigned long long seen[2] = {0, 0};
+  if ((e = cudaMemcpyAsync(c + 1, offsets + nq, 8, cudaMemcpyDeviceToDevice, s)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(seen, c, sizeof(seen), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+      (e = cudaStreamSynchronize(s)) != cudaSuccess)
+    return cuda_fail(e, "radius count");
+  hits.total = seen[1];
+  if (keep && seen[0] <= hits.rec.cap) hits.recorded = seen[0];
+  return KGPU_OK;
+}
+
+int radius_fill_kept(const DeviceTree& dt, QueryLaunch& q, const uint64_t* offsets,
+                     const kgpu_hits& hits) {
+  cudaStream_t s = q.stream;
+  cudaError_t e;
+  const bool f64 = dt.dtype == KGPU_F64;
+  q.capacity = hits.total;
+  if (hits.recorded != ~uint64_t(0)) {
+    e = f64 ? launch_place_hits<double>(q, offsets, hits.rec, hits.recorded)
+            : launch_place_hits<float>(q, offsets, hits.rec, hits.recorded);
+  } else {
+    e = with_walk_counter(q, [&](const QueryLaunch& qw) {
+      return f64 ? launch_within_fill<double>(dt, qw, offsets)
+                 : launch_within_fill<float>(dt, qw, offsets);
+    });
+  }
+  if (e != cudaSuccess) return cuda_fail(e, "launching the fill kernel");
+  if (!q.sorted) return KGPU_OK;
+  const size_t sa = f64 ? 8 : 4;
+  DevBuf sd, si;
+  if ((e = sd.alloc(hits.total * sa, s)) != cudaSuccess ||
+      (e = si.alloc(hits.total * 4, s)) != cudaSuccess)
+    return set_error(KGPU_ENOMEM, "device allocation failed");
+  e = f64 ? launch_seg_sort<double>(offsets, q.nq, hits.total, static_cast<double*>(q.out_d),
+                                    q.out_i, sd.as<double>(), si.as<uint32_t>(), s)
+          : launch_seg_sort<float>(offsets, q.nq, hits.total, static_cast<float*>(q.out_d),
+                                   q.out_i, sd.as<float>(), si.as<uint32_t>(), s);
+  return e == cudaSuccess ? KGPU_OK : cuda_fail(e, "launching the segmented sort");
+}
+
+namespace {
+// The description of a radius batch over one tree with device buffers.
+QueryLaunch radius_launch(const DeviceTree& dt, const kgpu_query_desc* d, const void* queries,
+                          uint64_t nq, cudaStream_t s) {
+  QueryLaunch q;
+  q.family = d->family;
+  q.metric = d->metric;
+  q.radius = d->radius;
+  q.exclusive = d->exclusive != 0;
+  q.sorted = d->family == KGPU_WITHIN && d->sorted != 0;
+  q.nq = nq;
+  apply_periodic(dt, d, q);
+  q.engine = engine_of(d->flags);
+  apply_tuning(d->tuning, q);
+  q.engine = engine_for(dt, q);
+  q.queries = queries;
+  q.stream = s;
+  return q;
+}
+}  // namespace
 }  // namespace kgpu
 
 extern "C" {
+
+int32_t kgpu_query_radius_count_keep(kgpu_tree* t, const kgpu_query_desc* d, const void* queries,
+                                     uint64_t nq, uint64_t* offsets, uint64_t* total,
+                                     kgpu_hits** out, void* stream) {
+  int st = check_query_desc(t, d, true);
+  if (st != KGPU_OK) return st;
+  if (d->flags & KGPU_FLAG_HOST_BUFFERS)
+    return set_error(KGPU_EINVAL, "kept hits take device pointers");
+  if (!offsets || !total || !out || (nq && !queries)) return set_error(KGPU_EINVAL, "NULL argument");
+  *out = nullptr;
+  const DeviceTree& dt = t->dt;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  QueryLaunch q = radius_launch(dt, d, queries, nq, s);
+  auto* h = new (std::nothrow) kgpu_hits();
+  if (!h) return set_error(KGPU_ENOMEM, "host allocation failed");
+  const cudaError_t e = maybe_spatial_order(dt, d, q, h->order, h->order_tmp, s);
+  h->ordered = q.order != nullptr;
+  st = e == cudaSuccess ? radius_count_keep(dt, q, offsets, *h) : cuda_fail(e, "ordering the batch");
+  if (st != KGPU_OK) {
+    delete h;
+    return st;
+  }
+  *total = h->total;
+  *out = h;
+  return KGPU_OK;
+}
+
+int32_t kgpu_query_radius_fill_kept(kgpu_tree* t, const kgpu_query_desc* d, const void* queries,
+                                    uint64_t nq, const uint64_t* offsets, const kgpu_hits* hits,
+                                    void* out_dists, uint32_t* out_items, void* stream) {
+  int st = check_query_desc(t, d, true);
+  if (st != KGPU_OK) return st;
+  if (!hits || !offsets || hits->nq != nq) return set_error(KGPU_EINVAL, "hits of another batch");
+  if (hits->counters.s != static_cast<cudaStream_t>(stream))
+    return set_error(KGPU_EINVAL, "hits are filled on the stream that counted them");
+  if (d->flags & KGPU_FLAG_HOST_BUFFERS)
+    return set_error(KGPU_EINVAL, "kept hits take device pointers");
+  if (hits->total == 0) return KGPU_OK;
+  if (!queries || !out_dists || !out_items) return set_error(KGPU_EINVAL, "NULL buffer");
+  QueryLaunch q = radius_launch(t->dt, d, queries, nq, static_cast<cudaStream_t>(stream));
+  q.out_d = out_dists;
+  q.out_i = out_items;
+  if (hits->ordered) q.order = hits->order.as<uint32_t>();
+  return radius_fill_kept(t->dt, q, offsets, *hits);
+}
+
+int32_t kgpu_hits_free(kgpu_hits* hits) {
+  delete hits;
+  return KGPU_OK;
+}
 
 int32_t kgpu_query(kgpu_tree* t, const kgpu_query_desc* d, const void* queries, uint64_t nq,
                    void* out_dists, uint32_t* out_items, uint32_t* out_counts, void* stream) {

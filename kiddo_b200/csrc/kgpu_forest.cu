@@ -21,6 +21,7 @@
 #include "../../include/kiddo_gpu.h"
 #include "kgpu_device.cuh"
 #include "kgpu_devbuf.h"
+#include "kgpu_hits.h"
 #include "kgpu_internal.h"
 #include "kgpu_launch.h"
 #include "kgpu_tree_impl.h"
@@ -284,6 +285,54 @@ int32_t kgpu_forest_query_radius_fill(kgpu_forest* f, const kgpu_query_desc* d,
     if (e != cudaSuccess) return cuda_err(e, "launching the segmented sort");
   }
   return KGPU_OK;
+}
+
+int32_t kgpu_forest_query_radius_count_keep(kgpu_forest* f, const kgpu_query_desc* d,
+                                            const void* queries, const uint32_t* tree_of,
+                                            const void* radii, uint64_t nq, uint64_t* offsets,
+                                            uint64_t* total, kgpu_hits** out, void* stream) {
+  QueryLaunch q;
+  int st = forest_launch(f, d, queries, tree_of, radii, nq, q, true);
+  if (st != KGPU_OK) return st;
+  if (!offsets || !total || !out) return set_error(KGPU_EINVAL, "NULL argument");
+  *out = nullptr;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  q.stream = s;
+  auto* h = new (std::nothrow) kgpu_hits();
+  if (!h) return set_error(KGPU_ENOMEM, "host allocation failed");
+  DevBuf work;
+  const cudaError_t e = nq ? prepare(f, d, q, work, h->order, h->order_tmp, s) : cudaSuccess;
+  h->ordered = q.order != nullptr;
+  st = e == cudaSuccess ? radius_count_keep(f->meta, q, offsets, *h)
+                        : cuda_err(e, "preparing the batch");
+  if (st != KGPU_OK) {
+    delete h;
+    return st;
+  }
+  *total = h->total;
+  *out = h;
+  return KGPU_OK;
+}
+
+int32_t kgpu_forest_query_radius_fill_kept(kgpu_forest* f, const kgpu_query_desc* d,
+                                           const void* queries, const uint32_t* tree_of,
+                                           const void* radii, uint64_t nq, const uint64_t* offsets,
+                                           const kgpu_hits* hits, void* out_dists,
+                                           uint32_t* out_items, void* stream) {
+  QueryLaunch q;
+  int st = forest_launch(f, d, queries, tree_of, radii, nq, q, true);
+  if (st != KGPU_OK) return st;
+  if (!hits || !offsets || hits->nq != nq) return set_error(KGPU_EINVAL, "hits of another batch");
+  if (hits->counters.s != static_cast<cudaStream_t>(stream))
+    return set_error(KGPU_EINVAL, "hits are filled on the stream that counted them");
+  if (hits->total == 0) return KGPU_OK;
+  if (!out_dists || !out_items) return set_error(KGPU_EINVAL, "NULL output buffer");
+  q.stream = static_cast<cudaStream_t>(stream);
+  q.out_d = out_dists;
+  q.out_i = out_items;
+  q.sorted = d->family == KGPU_WITHIN && d->sorted != 0;
+  if (hits->ordered) q.order = hits->order.as<uint32_t>();
+  return radius_fill_kept(f->meta, q, offsets, *hits);
 }
 
 // ---- CUDA graphs ------------------------------------------------------------

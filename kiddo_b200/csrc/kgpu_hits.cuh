@@ -1,0 +1,182 @@
+// kgpu_hits.cuh — radius queries in one walk: the counting pass keeps where its
+// hits are, and the filling pass places them from that.
+//
+// The two-pass form walks every tree twice, though the second walk only finds
+// again what the first one saw.  Here the counting pass (k_twithin_record)
+// appends a record per leaf chunk that holds hits: the chunk's address, the
+// mask of its points within the radius, the query and the hits it had before.
+// k_place_hits then takes a record per warp, recomputes the distances of the
+// masked points (the same operations, the same bits) and writes them at the
+// query's offset.  Records cost 20 bytes per 32 points with a hit; a batch with
+// more than its buffer holds is filled by the second walk instead.
+//
+// What bounds it: the placing pass is latency (record -> offset, query and rows
+// -> stores) hidden by four records per warp and the occupancy.
+#pragma once
+
+#include "kgpu_kernels.cuh"
+
+namespace kgpu {
+
+// CWithin's counting leaf scan, appending records.  A warp takes room for
+// kBatch records at a time, so most appends touch no shared counter.
+template <typename A, int K, typename M, bool kExclusive>
+struct CWithinRecord {
+  static constexpr bool kPruneOnEqual = kExclusive;
+  static constexpr uint32_t kBatch = 64;
+  A radius;
+  uint64_t count;
+  HitRecords rec;
+  unsigned long long at;  // the warp's next record
+  uint32_t left;          // of the room it took
+  __device__ explicit CWithinRecord(const HitRecords& r)
+      : radius(A(0)), count(0), rec(r), at(0), left(0) {}
+  __device__ __forceinline__ A max_dist() const { return radius; }
+  __device__ __forceinline__ bool unbounded_start() const { return radius == inf_of<A>(); }
+
+  __device__ __forceinline__ void leaf(int o, uint64_t qo, const CoopLeaf<A, K>& L, int lane) {
+    uint64_t cnt = shfl64(count, o);
+    const A orad = shfl(radius, o);
+    for (uint32_t c0 = 0; c0 < L.len; c0 += 32) {
+      const uint32_t p = c0 + lane;
+      bool pass = false;
+      if (p < L.len) {
+        uint32_t it;
+        const A d = coop_point<A, K>(L, p, it, CartesianDist<A, K, M>());
+        pass = kExclusive ? (d < orad) : (d <= orad);
+      }
+      const unsigned m = __ballot_sync(FULL, pass);
+      if (!m) continue;
+      if (left == 0) {
+        if (lane == 0) at = atomicAdd(rec.count, (unsigned long long)kBatch);
+        at = __shfl_sync(FULL, at, 0);
+        left = kBatch;
+      }
+      if (lane == 0 && at < rec.cap) {
+        const uint64_t rows = reinterpret_cast<uint64_t>(L.base) + c0 * row_bytes<A>();
+        rec.leaf[at] = make_uint4(uint32_t(rows), uint32_t(rows >> 32), m, uint32_t(cnt));
+        rec.query[at] = uint32_t(qo);
+      }
+      ++at;
+      --left;
+      cnt += uint64_t(__popc(m));
+    }
+    if (lane == o) count = cnt;
+  }
+  // Room taken and not used is left as empty records.
+  __device__ __forceinline__ void close(int lane) {
+    for (uint32_t j = lane; j < left; j += 32)
+      if (at + j < rec.cap) rec.leaf[at + j] = make_uint4(0, 0, 0, 0);
+  }
+};
+
+template <typename A, int K, typename M, bool EXCL>
+__global__ void __launch_bounds__(256) k_twithin_record(TreeView<A> tv0, Batch<A> b, A radius0,
+                                                        uint64_t* __restrict__ counts,
+                                                        HitRecords rec) {
+  static_assert(RowLeaves<A, K>::value, "records name rows");
+  extern __shared__ __align__(16) unsigned char tsmem[];
+  A* slot = reinterpret_cast<A*>(tsmem) + threadIdx.x;
+  const int stride = blockDim.x, lane = threadIdx.x & 31;
+  TravStats st;
+  CWithinRecord<A, K, M, EXCL> pol(rec);
+  ThreadWalk<A, K, M> wk;
+  coop_drive<A, K, M>(
+      tv0, b, wk, pol, slot, stride, st,
+      [&](uint64_t qi, const TreeView<A>&) {
+        pol.radius = b.radius(radius0, qi);
+        pol.count = 0;
+        return true;
+      },
+      [&](int w, uint64_t qo) {
+        const uint64_t cnt = shfl64(pol.count, w);
+        if (lane == 0) counts[qo] = cnt;
+      });
+  pol.close(lane);
+}
+
+// The records' hits at their queries' offsets: a warp takes kRecords records,
+// loads what all of them name and then writes them.
+template <typename A, int K, typename M>
+__global__ void __launch_bounds__(256) k_place_hits(const A* __restrict__ Q,
+                                                    const uint64_t* __restrict__ offsets,
+                                                    HitRecords rec, uint64_t n,
+                                                    A* __restrict__ out_d,
+                                                    uint32_t* __restrict__ out_i) {
+  constexpr int kRecords = 4;
+  const int lane = threadIdx.x & 31;
+  const uint64_t warps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
+  const unsigned below_me = (1u << lane) - 1u;
+  for (uint64_t r0 = ((uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * kRecords; r0 < n;
+       r0 += warps * kRecords) {
+    uint4 leaf[kRecords];
+    uint32_t query[kRecords];
+#pragma unroll
+    for (int j = 0; j < kRecords; ++j) {
+      leaf[j] = make_uint4(0, 0, 0, 0);
+      query[j] = 0;
+      if (r0 + j < n) {
+        leaf[j] = __ldg(rec.leaf + r0 + j);
+        if (leaf[j].z) query[j] = __ldg(rec.query + r0 + j);
+      }
+    }
+    A c[kRecords][K], q[kRecords][K];
+    uint32_t item[kRecords];
+    uint64_t to[kRecords];
+#pragma unroll
+    for (int j = 0; j < kRecords; ++j) {
+      if (!leaf[j].z) continue;
+      to[j] = __ldg(offsets + query[j]) + leaf[j].w;
+#pragma unroll
+      for (int d = 0; d < K; ++d) q[j][d] = __ldg(Q + uint64_t(query[j]) * K + d);
+      const uint8_t* rows =
+          reinterpret_cast<const uint8_t*>(uint64_t(leaf[j].y) << 32 | leaf[j].x);
+      if ((leaf[j].z >> lane) & 1u) load_row<A, K>(rows, lane, c[j], item[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < kRecords; ++j) {
+      if ((leaf[j].z >> lane) & 1u) {
+        const uint64_t w = to[j] + __popc(leaf[j].z & below_me);
+        out_d[w] = point_dist<M, A, K>(c[j], q[j]);
+        out_i[w] = item[j];
+      }
+    }
+  }
+}
+
+template <typename A>
+cudaError_t launch_within_record(const DeviceTree& t, const QueryLaunch& q, uint64_t* counts,
+                                 const HitRecords& rec) {
+  const TreeView<A> tv = make_view<A>(t);
+  const Batch<A> b = make_batch<A>(q, kRefillCoop);
+  return with_metric(q.metric, [&](auto m) {
+    using M = decltype(m);
+    return with_excl(q.exclusive, [&](auto ex) -> cudaError_t {
+      constexpr bool EX = decltype(ex)::value;
+      const size_t smem = size_t(t.max_stem_level + 2) * 256 * sizeof(A);
+      auto kern = k_twithin_record<A, 3, M, EX>;
+      const cudaError_t e =
+          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+      if (e != cudaSuccess) return e;
+      kern<<<grid_for(kern, smem, (q.nq + 31) / 32), 256, smem, q.stream>>>(tv, b, A(q.radius),
+                                                                            counts, rec);
+      g_launches++;
+      return cudaGetLastError();
+    });
+  });
+}
+
+template <typename A>
+cudaError_t launch_place_hits(const QueryLaunch& q, const uint64_t* offsets, const HitRecords& rec,
+                              uint64_t n) {
+  if (n == 0) return cudaSuccess;
+  return with_metric(q.metric, [&](auto m) {
+    auto kern = k_place_hits<A, 3, decltype(m)>;
+    kern<<<grid_for(kern, 0, (n + 3) / 4), 256, 0, q.stream>>>(
+        static_cast<const A*>(q.queries), offsets, rec, n, static_cast<A*>(q.out_d), q.out_i);
+    g_launches++;
+    return cudaGetLastError();
+  });
+}
+
+}  // namespace kgpu

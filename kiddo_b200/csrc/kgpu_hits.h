@@ -1,0 +1,27 @@
+// kgpu_hits.h — what a counting pass keeps for the filling pass (kgpu_hits).
+#pragma once
+
+#include <cstdint>
+
+#include "kgpu_devbuf.h"
+#include "kgpu_launch.h"
+
+// The processing order and, where the counting pass recorded them, the places
+// of a batch's hits; all on the stream of the counting call.
+struct kgpu_hits {
+  kgpu::DevBuf order, order_tmp, leaf, query, counters;
+  kgpu::HitRecords rec;
+  bool ordered = false;
+  uint64_t recorded = ~uint64_t(0);  // records to place; ~0: none were kept, or not all
+  uint64_t nq = 0, total = 0;
+};
+
+namespace kgpu {
+// Counts every query's hits, scans them into offsets[0..nq] and keeps what the
+// fill needs; `q` describes the batch (order included in `hits`).  Waits for
+// the total.  Returns a kgpu_status.
+int radius_count_keep(const DeviceTree& dt, QueryLaunch& q, uint64_t* offsets, kgpu_hits& hits);
+// Writes and (q.sorted) sorts the hits.
+int radius_fill_kept(const DeviceTree& dt, QueryLaunch& q, const uint64_t* offsets,
+                     const kgpu_hits& hits);
+}  // namespace kgpu

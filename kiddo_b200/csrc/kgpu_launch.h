@@ -171,6 +171,20 @@ template <typename A> cudaError_t launch_within_count(const DeviceTree& t, const
                                                        uint64_t* counts);
 template <typename A> cudaError_t launch_within_fill(const DeviceTree& t, const QueryLaunch& q,
                                                       const uint64_t* offsets);
+// Records of the hits that a counting pass saw (kgpu_hits.cuh): per leaf chunk
+// with hits its rows' address, the mask of hits and the hits of its query before
+// it, and the query.  `count` may pass `cap`; records beyond are lost.
+struct HitRecords {
+  uint4* leaf = nullptr;
+  uint32_t* query = nullptr;
+  unsigned long long* count = nullptr;
+  uint64_t cap = 0;
+};
+// 3-D arithmetic trees (rows, ThreadWalk), no periodic box.
+template <typename A> cudaError_t launch_within_record(const DeviceTree& t, const QueryLaunch& q,
+                                                       uint64_t* counts, const HitRecords& rec);
+template <typename A> cudaError_t launch_place_hits(const QueryLaunch& q, const uint64_t* offsets,
+                                                    const HitRecords& rec, uint64_t n);
 // Processing order grouped by straight-descent leaf.  `scratch` must hold
 // spatial_order_scratch_bytes(t, nq) bytes; order[nq] receives query indices.
 size_t spatial_order_scratch_bytes(const DeviceTree& t, const QueryLaunch& q);
