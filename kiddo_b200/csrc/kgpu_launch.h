@@ -103,40 +103,51 @@ inline void apply_tuning(uint32_t tuning, QueryLaunch& q) {
 
 // The engine of a batch that asks for none: small batches of 2-D and 3-D trees
 // take the warp engine.  A thread walks its query alone, so a batch too small
-// to fill the GPU with threads takes as long as one thread's walk (0.1 to 1
+// to fill the GPU with threads takes as long as one thread's walk (50 us to 1
 // ms); a warp answers a query in about a twentieth of that, and the engines
-// meet where the warps' throughput limit reaches the thread's latency.
-// Measured, 1M-point uniform and clustered trees and 10k points (thread / warp
-// engine, us, both sides of the line): nearest_one f32 32768 queries 129 / 84,
-// 65535 145 / 146; nearest_n f32 k = 8 65535 305 / 286, 98304 331 / 436; k = 16
-// 65535 468 / 371, 98304 505 / 556; k = 32 98304 1064 / 781, 131072 1093 / 1024,
-// 262144 1824 / 2012; best_n 65535 308 / 234, 98304 341 / 348; within 49152 560
-// / 451, 65536 541 / 587; periodic within f64 32768 1049 / 904, 49152 1069 /
-// 1217.  Periodic lists (65535 queries: f32 k = 8 836 / 591, f64 k = 16 1445 /
-// 1190) end where the plain-walk path begins (kgpu_periodic_fast.cu).  f64 lists above 32 entries are the warp engine's at every size
-// (393216 queries: k = 40 9319 / 8491, k = 64 18620 / 12521): the per-thread
-// lists leave two blocks per SM.  Explicit engines, Donnelly and Mapped trees
-// (thread walks only) and lists kept in output rows are not touched.
+// meet where the warps' throughput reaches the thread's latency: earlier over
+// uniform points, later over clustered ones, whose slowest walks are longer.
+// The lines lie between.  Measured, 1M-point trees, uniform; clustered (thread
+// or cooperative / warp engine, us):
+//   nearest_one f32 24576 queries 73/68; 127/66, 49152 79/125; 129/105
+//   nearest_n f32 k = 8 32768 131/153; 360/185, 49152 137/220; 372/239
+//     k = 16 32768 198/198; 473/233, 65535 217/366; 500/394
+//     k = 32 40000 376/332; 434/386, 65535 384/537; 455/565
+//   nearest_n f64 k = 16 40000 335/294; 382/274, 65535 345/458; 406/432
+//     k = 32 49152 540/495; 583/481, 65535 546/639; 587/605
+//   best_n f32 40000 155/147; 126/106, 49152 156/175; 132/128
+//   within f32 3-D (one walk) 16384 239/242; 200/190, 24576 242/286; 202/225,
+//     2-D (two walks) 40000 287/276
+//   periodic nearest_n f32 k = 16 32768 369/370; 468/388, f64 k = 32 24576
+//     766/593; 913/632, 32768 772/798; 911/803; within f32 24576 439/441;
+//     354/308, f64 16384 567/530; 412/379
+//   f32 k = 64 49152 1164/1334; 1871/1402
+// f64 lists above 32 entries are the warp engine's at every size (49152
+// queries: k = 40 1907/1138, k = 64 3747/1719): the per-thread lists leave two
+// blocks per SM.  Explicit engines, Donnelly and Mapped trees (thread walks
+// only) and lists kept in output rows are not touched.
 inline int engine_for(const DeviceTree& t, const QueryLaunch& q) {
   if (q.engine != 0 || t.scalar_walk() || (t.dims != 2 && t.dims != 3)) return q.engine;
   const uint64_t k = uint64_t(q.k > 0 ? q.k : 1);
+  const bool f64 = t.dtype == KGPU_F64;
   uint64_t below = 0;
   switch (q.family) {
     case KGPU_NEAREST_ONE:
-      below = 40960;
+      below = 28672;
       break;
     case KGPU_NEAREST_N:
     case KGPU_NEAREST_N_WITHIN:
-      if (q.periodic) below = k <= 32 ? 65536 : 0;
-      else if (k <= 32) below = 40960 + 2560 * k;
-      else below = t.dtype == KGPU_F64 ? ~uint64_t(0) : 65536;
+      if (q.periodic) below = k <= 32 ? (f64 ? 22528 : 28672) + 384 * k : 0;
+      else if (k > 32) below = f64 ? ~uint64_t(0) : 32768 + 512 * (k - 32);
+      else if (k > (f64 ? 13 : 20)) below = f64 ? 57344 : 49152;
+      else below = 32768 + 768 * k;
       break;
     case KGPU_BEST_N_WITHIN:
-      below = 81920;
+      below = 40960;
       break;
     case KGPU_WITHIN:
     case KGPU_WITHIN_UNSORTED:
-      below = q.periodic ? 40960 : 57344;
+      below = q.periodic ? (f64 ? 18432 : 24576) : t.dims == 3 ? 16384 : 40960;
       break;
     default:  // approx: one leaf per query, the thread engine's at every size
       break;

@@ -22,22 +22,25 @@ def _same(a, b, label):
         assert x.tobytes() == y.tobytes(), f"{label}: {f} differs"
 
 
-def _families(dims, r):
+def _families(dtype, dims, r):
     box = np.ones(dims)
+    f64 = dtype == np.float64
     return {
-        "one": (40960, lambda b: b.nearest_one(SE)),
-        "one_manhattan": (40960, lambda b: b.nearest_one(MAN)),
-        "n5": (53760, lambda b: b.nearest_n(SE, 5)),
-        "n16_unsorted": (81920, lambda b: b.nearest_n(CHEB, 16).unsorted()),
-        "n32_within_excl": (122880,
+        "one": (28672, lambda b: b.nearest_one(SE)),
+        "one_manhattan": (28672, lambda b: b.nearest_one(MAN)),
+        "n5": (36608, lambda b: b.nearest_n(SE, 5)),
+        "n16_unsorted": (57344 if f64 else 45056, lambda b: b.nearest_n(CHEB, 16).unsorted()),
+        "n32_within_excl": (57344 if f64 else 49152,
                             lambda b: b.nearest_n(SE, 32).within(r).exclusive_boundaries()),
-        "n40": (65536, lambda b: b.nearest_n(SE, 40)),
-        "best7": (81920, lambda b: b.best_n_within(SE, r, 7)),
-        "within": (57344, lambda b: b.within(SE, r)),
-        "within_unsorted_excl": (57344,
+        "n40": (36864, lambda b: b.nearest_n(SE, 40)),
+        "best7": (40960, lambda b: b.best_n_within(SE, r, 7)),
+        "within": (16384 if dims == 3 else 40960, lambda b: b.within(SE, r)),
+        "within_unsorted_excl": (16384 if dims == 3 else 40960,
                                  lambda b: b.within(MAN, r).unsorted().exclusive_boundaries()),
-        "periodic_n9": (65536, lambda b: b.periodic_boundary_condition(box).nearest_n(SE, 9)),
-        "periodic_within": (40960, lambda b: b.periodic_boundary_condition(box).within(SE, r)),
+        "periodic_n9": ((22528 if f64 else 28672) + 3456,
+                        lambda b: b.periodic_boundary_condition(box).nearest_n(SE, 9)),
+        "periodic_within": (18432 if f64 else 24576,
+                            lambda b: b.periodic_boundary_condition(box).within(SE, r)),
     }
 
 
@@ -51,7 +54,7 @@ def test_default_engine_gives_the_thread_engines_bytes(dtype, dims):
     P = rng.random((5_001, dims)).astype(dtype)
     P[100:140] = P[100]                       # equal distances
     tree = kb.ImmutableKdTree.new_from_slice(P)
-    for name, (line, make) in _families(dims, 2e-3 if dims == 3 else 4e-4).items():
+    for name, (line, make) in _families(dtype, dims, 2e-3 if dims == 3 else 4e-4).items():
         Q = rng.random((line + 1, dims)).astype(dtype)
         Q[5::1009] = P[(np.arange(len(Q[5::1009])) * 7) % len(P)]
         Q[11::4001] = np.nan
