@@ -91,9 +91,10 @@ def _vp(a: np.ndarray):
 
 def _host_array(shape, dtype):
     """Result buffer in pinned host memory when torch can provide it (the
-    library then copies results back at full bus speed), else pageable."""
+    library then copies results back at full bus speed, and without a staging
+    copy), else pageable; a few KB are not worth a pinned block."""
     n = int(np.prod(shape))
-    if n * np.dtype(dtype).itemsize >= (1 << 20):
+    if n * np.dtype(dtype).itemsize >= (1 << 14):
         try:
             import torch
             if torch.cuda.is_available():

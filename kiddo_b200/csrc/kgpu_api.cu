@@ -894,26 +894,31 @@ __global__ void k_short_rows(const uint32_t* __restrict__ counts, uint64_t n, ui
 #define KGPU_HOST_SLOTS 3
 #endif
 #ifndef KGPU_HOST_CHUNK_LOG2
-#define KGPU_HOST_CHUNK_LOG2 21
+#define KGPU_HOST_CHUNK_LOG2 19
 #endif
 #ifndef KGPU_HOST_EDGE_DIV
 #define KGPU_HOST_EDGE_DIV 8
 #endif
-// Host buffers: the batch goes through in 2M-query chunks on three internal
-// streams, each with its own device buffers, so the copy of one chunk's
-// queries in, another chunk's kernel and a third chunk's results out run at
-// the same time (full overlap needs pinned host memory).  With two slots a
+// Host buffers: a batch of 2^20 queries or more goes through in chunks of 2^19
+// on three internal streams, each with its own device buffers, so the copy of
+// one chunk's queries in, another chunk's kernel and a third chunk's results out
+// run at the same time (full overlap needs pinned host memory).  With two slots a
 // chunk's kernel waited for the results of the chunk two back to leave its
-// buffers; on kNN16 over 16M queries, three slots took the call from 55.8 to
-// 49.1 ms, against 36.9 ms for the result copy alone.  Work already queued on
-// the caller's stream runs first; the call returns when every result is on
-// the host.
+// buffers.  kNN16 (pinned, 128 result bytes a query): 2M queries 9.83 ms in one
+// piece, 8.25 in chunks of 2^18, 7.81 of 2^19; 8M queries 27.85 ms in chunks of
+// 2^21, 26.77 of 2^18, 23.03 of 2^19, against 17.9 ms for the result copy alone.
+// A smaller batch is one chunk on the caller's own stream: making streams, events
+// and a second set of buffers cost more than the overlap gave (500k queries 3.15
+// ms either way; 5,000 queries 284 us with streams and pageable results, 140
+// without and with pinned ones).  Work already queued on the caller's stream runs first; the call returns when every result is
+// on the host.
 int query_host_pipelined(const DeviceTree& dt, const kgpu_query_desc* d, const QueryLaunch& base,
                          const void* queries, uint64_t nq, int w, void* out_dists,
                          uint32_t* out_items, uint32_t* out_counts, cudaStream_t s) {
   const size_t sa = dt.dtype == KGPU_F64 ? 8 : 4;
   constexpr int kSlots = KGPU_HOST_SLOTS;
-  const uint64_t chunk = std::min<uint64_t>(nq, uint64_t(1) << KGPU_HOST_CHUNK_LOG2);
+  constexpr uint64_t kChunk = uint64_t(1) << KGPU_HOST_CHUNK_LOG2;
+  const uint64_t chunk = nq < 2 * kChunk ? nq : kChunk;
   const int nslots = int(std::min<uint64_t>(kSlots, (nq + chunk - 1) / chunk));
   cudaStream_t st[kSlots] = {};
   // nearest_n without a radius fills min(k, size) entries in every row whose
@@ -922,7 +927,7 @@ int query_host_pipelined(const DeviceTree& dt, const kgpu_query_desc* d, const Q
   // on the device (all_counts), a small kernel counts each chunk's rows short
   // of that, and only chunks with such rows are copied back at the end.
   uint32_t* const host_counts = out_counts;
-  const bool counts_known = out_counts && d->family == KGPU_NEAREST_N;
+  const bool counts_known = out_counts && d->family == KGPU_NEAREST_N && nslots > 1;
   const uint32_t full = uint32_t(std::min<uint64_t>(uint64_t(w), dt.size));
   const uint64_t edge = std::max<uint64_t>(1, chunk / KGPU_HOST_EDGE_DIV);
   const uint64_t max_chunks = (nq + edge - 1) / edge + 1;
@@ -942,9 +947,13 @@ int query_host_pipelined(const DeviceTree& dt, const kgpu_query_desc* d, const Q
     return cudaGetLastError();
   };
   cudaEvent_t ready = nullptr;
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventRecord(ready, s);
-  for (int i = 0; i < nslots && e == cudaSuccess; ++i) {
+  if (nslots == 1) {
+    st[0] = s;
+  } else if (e == cudaSuccess) {
+    if ((e = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming)) == cudaSuccess)
+      e = cudaEventRecord(ready, s);
+  }
+  for (int i = 0; i < nslots && nslots > 1 && e == cudaSuccess; ++i) {
     e = cudaStreamCreateWithFlags(&st[i], cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(st[i], ready, 0);
   }
@@ -963,7 +972,7 @@ int query_host_pipelined(const DeviceTree& dt, const kgpu_query_desc* d, const Q
     // The first and the last chunk are short (an eighth of a chunk): the first
     // chunk's kernel runs before any result can leave, and the last chunk's
     // results leave after every kernel, so shorter ends shorten the
-    // unoverlapped head and tail (kNN16 over 16M queries: 50.9 -> 47.1 ms).
+    // unoverlapped head and tail.
     auto chunk_len = [&](uint64_t c0) -> uint64_t {
       const uint64_t rem = nq - c0;
       if (nslots == 1 || rem <= edge) return rem;
@@ -1015,7 +1024,8 @@ int query_host_pipelined(const DeviceTree& dt, const kgpu_query_desc* d, const Q
     }
     if (counts_known && status == KGPU_OK) std::fill(host_counts, host_counts + nq, full);
     for (int i = 0; i < nslots; ++i)
-      if (st[i] && (e = cudaStreamSynchronize(st[i])) != cudaSuccess && status == KGPU_OK)
+      if ((st[i] || nslots == 1) && (e = cudaStreamSynchronize(st[i])) != cudaSuccess &&
+          status == KGPU_OK)
         status = cuda_fail(e, "query execution");
     if (counts_known && status == KGPU_OK) {
       // the chunks with short rows, if any, bring their counts back
@@ -1028,7 +1038,7 @@ int query_host_pipelined(const DeviceTree& dt, const kgpu_query_desc* d, const Q
       if (e != cudaSuccess) status = cuda_fail(e, "copying results to the host");
     }
   }  // device buffers are released on their streams here
-  for (int i = 0; i < nslots; ++i)
+  for (int i = 0; i < nslots && nslots > 1; ++i)
     if (st[i]) {
       cudaStreamSynchronize(st[i]);
       cudaStreamDestroy(st[i]);
