@@ -37,6 +37,7 @@ CU_SOURCES = ["kgpu_api.cu", "kgpu_scan.cu", "kgpu_segsort.cu", "kgpu_noalloc.cu
               "kernels_f64_radius.cu",
               "kernels_f32_rows.cu",
               "kernels_f64_rows.cu",
+              "kernels_approx.cu",
               "kernels_f32_hits.cu",
               "kernels_f64_hits.cu",
               ]

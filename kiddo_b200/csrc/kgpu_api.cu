@@ -839,6 +839,8 @@ cudaError_t launch_fixed(const DeviceTree& t, const QueryLaunch& q) {
                       (!q.periodic || q.family != KGPU_NEAREST_ONE || t.scalar_walk()) && !big_k;
   // the warp engine keeps its fixed shares: it takes one query at a time
   if (!thread) return launch_wfixed<A>(t, q);
+  // a batch in the caller's order: warp-wide leaf scans, even shares, no counter
+  if (q.family == KGPU_APPROX_NEAREST_ONE && !q.order) return launch_approx<A>(t, q);
   return with_work_counter(q, [&](const QueryLaunch& qw) { return launch_tfixed<A>(t, qw); });
 }
 template cudaError_t launch_fixed<float>(const DeviceTree&, const QueryLaunch&);
@@ -851,7 +853,8 @@ namespace {
 // hand the kernels that processing order (same results, better locality).
 cudaError_t maybe_spatial_order(const DeviceTree& dt, const kgpu_query_desc* d, QueryLaunch& q,
                                 DevBuf& ob, DevBuf& sb, cudaStream_t s) {
-  if (!want_spatial_order(d->flags, q.nq, q.forest ? q.total_leaves : dt.leaf_count))
+  if (!want_spatial_order(d->flags, q.nq, q.forest ? q.total_leaves : dt.leaf_count) ||
+      !order_pays(dt, q, d->flags))
     return cudaSuccess;
   cudaError_t e;
   if ((e = ob.alloc(q.nq * 4, s)) != cudaSuccess) return e;

@@ -155,6 +155,17 @@ inline int engine_for(const DeviceTree& t, const QueryLaunch& q) {
   return q.nq < below ? 1 : q.engine;
 }
 
+// Whether a large batch that does not ask for leaf-grouped order gets it.  Not
+// f32 approx: a leaf is one 480-byte read there, and reading it again for each
+// query costs less than the sort and the scattered queries and results (16M
+// queries of a 16M-point tree 1.71 ms against 2.72, 8M of 100k points 0.55
+// against 0.99, 2-D 8M of 8M 0.95 against 1.11).  f64 leaves are twice that and
+// do not (8M of 8M 1.58 against 1.28 ms, 2-D 4M of 4M 0.60 against 0.55).
+inline bool order_pays(const DeviceTree& t, const QueryLaunch& q, uint32_t flags) {
+  return (flags & KGPU_FLAG_SPATIAL_ORDER) || q.family != KGPU_APPROX_NEAREST_ONE ||
+         t.dtype == KGPU_F64 || q.engine == 1 || (t.dims != 2 && t.dims != 3);
+}
+
 // Fixed-size families: dispatches to the thread engine (2-D/3-D trees) or the
 // warp engine (everything else, periodic included).
 template <typename A> cudaError_t launch_fixed(const DeviceTree& t, const QueryLaunch& q);
@@ -167,6 +178,9 @@ template <typename A>
 cudaError_t periodic_fast(const DeviceTree& t, const QueryLaunch& q, bool& handled);
 template <typename A> cudaError_t launch_wfixed(const DeviceTree& t, const QueryLaunch& q);
 template <typename A> cudaError_t launch_tfixed(const DeviceTree& t, const QueryLaunch& q);
+// approx nearest_one on 2-D and 3-D trees of either stem order, queries in the
+// caller's order (kernels_approx.cu).
+template <typename A> cudaError_t launch_approx(const DeviceTree& t, const QueryLaunch& q);
 // Lists of any length held in the output rows (kernels_*_rows.cu).
 template <typename A> cudaError_t launch_trow(const DeviceTree& t, const QueryLaunch& q);
 // Donnelly-stem kernels, defined in their own translation units
