@@ -1032,6 +1032,28 @@ __global__ void k_leaf_rows_to_tiles(const uint8_t* __restrict__ rows, uint8_t* 
   }
 }
 
+// Least item of every leaf, one warp per leaf (best_n_within leaves out leaves
+// whose items are all too high).
+template <typename A, int K>
+__global__ void k_leaf_min(const uint8_t* __restrict__ arena, const uint2* __restrict__ extents,
+                           uint64_t leaves, uint32_t* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  for (uint64_t l = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; l < leaves;
+       l += (uint64_t(gridDim.x) * blockDim.x) >> 5) {
+    const uint2 ex = extents[l];
+    const uint8_t* leaf = arena + size_t(ex.x) * 8;
+    uint32_t least = 0xffffffffu;
+    for (uint32_t p = lane; p < ex.y; p += 32) {
+      uint32_t off, w, i;
+      tile_slot<A, K>(ex.y, p, off, w, i);
+      least = min(least,
+                  reinterpret_cast<const uint32_t*>(leaf + off + K * w * sizeof(A))[i]);
+    }
+    least = __reduce_min_sync(FULL, least);
+    if (lane == 0) out[l] = least;
+  }
+}
+
 inline unsigned blocks_for(uint64_t n, unsigned threads = 256) {
   const uint64_t b = (n + threads - 1) / threads;
   return unsigned(std::max<uint64_t>(1, std::min<uint64_t>(b, 148ull * 64)));
@@ -1253,6 +1275,8 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
        (e = scratch_alloc(reinterpret_cast<void**>(&dt.arena), dev_bytes + 16, s)) !=
            cudaSuccess) ||
       (e = scratch_alloc(&dt.extents, std::max<size_t>(16, leaves * 8), s)) != cudaSuccess ||
+      (e = scratch_alloc(reinterpret_cast<void**>(&dt.leaf_min),
+                         std::max<size_t>(16, leaves * 4), s)) != cudaSuccess ||
       (moved && (e = scratch_alloc(&dt.src_extents, std::max<size_t>(16, leaves * 8), s)) !=
                     cudaSuccess))
     return cuda_fail_b(e, "tree arrays");
@@ -1270,14 +1294,34 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
       g_launches++;
     }
   }
-  if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess)
+  if ((e = cudaGetLastError()) != cudaSuccess || (e = fill_leaf_min(dt, s)) != cudaSuccess ||
+      (e = cudaStreamSynchronize(s)) != cudaSuccess)
     return cuda_fail_b(e, "writing the leaves");
   dt.device_bytes = std::max<size_t>(16, stem_count * sizeof(A)) + dev_bytes + 16 +
-                    leaves * 8 * (moved ? 2 : 1);
+                    leaves * (8 * (moved ? 2 : 1) + 4);
   return KGPU_OK;
 }
 
 }  // namespace
+
+cudaError_t fill_leaf_min(const DeviceTree& dt, cudaStream_t s) {
+  if (dt.leaf_count == 0) return cudaSuccess;
+  const unsigned grid = blocks_for(uint64_t(dt.leaf_count) * 32);
+  auto run = [&](auto kern) {
+    kern<<<grid, 256, 0, s>>>(dt.arena, static_cast<const uint2*>(dt.extents), dt.leaf_count,
+                              dt.leaf_min);
+    g_launches++;
+    return cudaGetLastError();
+  };
+  const bool f64 = dt.dtype == KGPU_F64;
+  switch (dt.dims) {
+    case 1: return f64 ? run(k_leaf_min<double, 1>) : run(k_leaf_min<float, 1>);
+    case 2: return f64 ? run(k_leaf_min<double, 2>) : run(k_leaf_min<float, 2>);
+    case 3: return f64 ? run(k_leaf_min<double, 3>) : run(k_leaf_min<float, 3>);
+    case 4: return f64 ? run(k_leaf_min<double, 4>) : run(k_leaf_min<float, 4>);
+  }
+  return cudaErrorInvalidValue;
+}
 
 cudaError_t convert_leaf_layout(const DeviceTree& dt, const uint8_t* src, uint8_t* dst,
                                 bool to_rows, cudaStream_t s) {

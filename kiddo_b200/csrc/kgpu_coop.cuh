@@ -82,6 +82,14 @@ struct CBestN {
   __device__ __forceinline__ void reset(A r) { n = 0; radius = r; last = 0; }
   __device__ __forceinline__ A max_dist() const { return radius; }
   __device__ __forceinline__ bool unbounded_start() const { return false; }
+  // A leaf whose items all lie at or above a full list's last changes nothing
+  // (its filter drops them whatever their distance): one load in the owner's
+  // lane instead of a scan by the warp (4M queries of 32 catalogues, n = 5: 7.08
+  // to 4.25 ms).
+  static constexpr bool kSkips = true;
+  __device__ __forceinline__ bool skip(const TreeView<A>& tv, uint32_t leaf) const {
+    return n == k && __ldg(tv.leaf_min + leaf) >= last;
+  }
 
   __device__ __forceinline__ void leaf(int o, uint64_t, const CoopLeaf<A, K>& L, int lane) {
     int nn = __shfl_sync(FULL, n, o);
@@ -326,6 +334,10 @@ struct CRowList {
   }
   __device__ __forceinline__ bool unbounded_start() const {
     return !BEST && radius == inf_of<A>();
+  }
+  static constexpr bool kSkips = true;  // as CBestN
+  __device__ __forceinline__ bool skip(const TreeView<A>& tv, uint32_t leaf) const {
+    return BEST && n == k && __ldg(tv.leaf_min + leaf) >= last;
   }
 
   __device__ __forceinline__ void leaf(int o, uint64_t qo, const CoopLeaf<A, K>& L, int lane) {

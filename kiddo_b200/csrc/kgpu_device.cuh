@@ -175,6 +175,7 @@ struct TreeView {
   const uint32_t* __restrict__ leaf_map;
   uint64_t map_min;
   uint32_t map_len;
+  const uint32_t* __restrict__ leaf_min;  // least item of each leaf
 };
 
 // resolve_terminal_stem (orchestrator/mod.rs:183-192) for Mapped trees: the
@@ -838,6 +839,8 @@ struct BestNPolicy {
     const uint32_t len = ex.y;
     const bool full_at_entry = n == k;
     const uint32_t thr_item = shfl(li, k - 1);
+    // every item of the leaf at or above the full list's last: none can enter
+    if (full_at_entry && __ldg(tv.leaf_min + l) >= thr_item) return len;
     for (uint32_t b = 0; b < len; b += 32) {
       const uint32_t p = b + lane;
       A dd = inf_of<A>();
@@ -941,6 +944,7 @@ struct BestNBigPolicy {
     const uint32_t len = ex.y;
     const bool full_at_entry = n == k;
     const uint32_t thr_item = full_at_entry ? li[k - 1] : 0u;
+    if (full_at_entry && __ldg(tv.leaf_min + l) >= thr_item) return len;
     for (uint32_t b = 0; b < len; b += 32) {
       const uint32_t p = b + lane;
       A dd = inf_of<A>();

@@ -324,6 +324,14 @@ __device__ __forceinline__ bool refill_lanes(const Batch<A>& b, LaneFeeder& fd, 
   return __any_sync(FULL, active);
 }
 
+// Policies that can tell from a leaf's number that nothing in it can enter
+// their list (skip(tv, leaf)) save the warp its scan; the leaf still counts as
+// visited, as in the reference's walk.
+template <typename Pol, typename = void>
+struct HasSkip : std::false_type {};
+template <typename Pol>
+struct HasSkip<Pol, std::void_t<decltype(Pol::kSkips)>> : std::true_type {};
+
 // ---------------------------------------------------------------------------
 // The driver: lane-refilled per-thread walks, cooperative leaf scans.
 //   start(qi, tv) sets the policy up for a fresh query in this lane and says
@@ -375,6 +383,7 @@ __device__ __forceinline__ void coop_drive(const TreeView<A>& tv0, const Batch<A
     }
     const uint8_t* lb = nullptr;
     uint32_t len = 0;
+    bool scan = true;  // whether the leaf could change the lane's result
     if (active) {
       const uint32_t leaf = wk.descend(tv, q, pol, bounded, slot, stride, st);
       const uint2 ex = wk.leaf_extents(tv, leaf);
@@ -382,8 +391,9 @@ __device__ __forceinline__ void coop_drive(const TreeView<A>& tv0, const Batch<A
       len = ex.y;
       st.points += len;
       ++st.leaves;
+      if constexpr (HasSkip<Pol>::value) scan = !pol.skip(tv, leaf);
     }
-    for (unsigned lm = __ballot_sync(FULL, active); lm; lm &= lm - 1) {
+    for (unsigned lm = __ballot_sync(FULL, active && scan); lm; lm &= lm - 1) {
       const int o = __ffs(lm) - 1;
       pol.leaf(o, shfl64(qi, o), coop_leaf<A, K>(o, lb, len, q), lane);
     }
