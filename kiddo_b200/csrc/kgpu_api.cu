@@ -170,7 +170,7 @@ void release_tree_arrays(DeviceTree& dt) {
     if (dt.arena) cudaFreeAsync(dt.arena, nullptr);
     if (dt.extents) cudaFreeAsync(dt.extents, nullptr);
     if (dt.src_extents) cudaFreeAsync(dt.src_extents, nullptr);
-    if (dt.leaf_min) cudaFreeAsync(dt.leaf_min, nullptr);
+    if (dt.item_min) cudaFreeAsync(dt.item_min, nullptr);
     cudaStreamSynchronize(nullptr);
     if (cur != dt.device) cudaSetDevice(cur);
   } else {
@@ -178,13 +178,13 @@ void release_tree_arrays(DeviceTree& dt) {
     cudaFree(dt.arena);
     cudaFree(dt.extents);
     cudaFree(dt.src_extents);
-    cudaFree(dt.leaf_min);
+    cudaFree(dt.item_min);
   }
   dt.stems = nullptr;
   dt.arena = nullptr;
   dt.extents = nullptr;
   dt.src_extents = nullptr;
-  dt.leaf_min = nullptr;
+  dt.item_min = nullptr;
 }
 
 }  // namespace kgpu
@@ -531,19 +531,18 @@ int create_tree(const kgpu_tree_desc* d, const kgpu_leaf_map* m, void* stream,
   if ((e = cudaMalloc(&dt.stems, stem_bytes)) != cudaSuccess ||
       (e = cudaMalloc(reinterpret_cast<void**>(&dt.arena), arena_bytes)) != cudaSuccess ||
       (e = cudaMalloc(&dt.extents, ex_bytes)) != cudaSuccess ||
-      (e = cudaMalloc(reinterpret_cast<void**>(&dt.leaf_min), std::max<size_t>(16, ex_bytes / 2))) !=
-          cudaSuccess ||
+      (e = cudaMalloc(reinterpret_cast<void**>(&dt.item_min), ex_bytes)) != cudaSuccess ||
       (moved && (e = cudaMalloc(&dt.src_extents, ex_bytes)) != cudaSuccess)) {
     cudaFree(dt.stems);
     cudaFree(dt.arena);
     cudaFree(dt.extents);
-    cudaFree(dt.leaf_min);
+    cudaFree(dt.item_min);
     cudaFree(dt.src_extents);
     delete t;
     if (e == cudaErrorMemoryAllocation) return set_error(KGPU_ENOMEM, "device allocation failed");
     return cuda_fail(e, "cudaMalloc");
   }
-  dt.device_bytes = stem_bytes + arena_bytes + ex_bytes * (moved ? 2 : 1) + ex_bytes / 2;
+  dt.device_bytes = stem_bytes + arena_bytes + ex_bytes * (moved ? 3 : 2);
   if (d->stem_count) e = cudaMemcpyAsync(dt.stems, d->stems, d->stem_count * sa, cudaMemcpyHostToDevice, s);
   // 3-D leaves are staged as tiles and re-encoded as rows on the device
   DevBuf tiles;
@@ -566,7 +565,7 @@ int create_tree(const kgpu_tree_desc* d, const kgpu_leaf_map* m, void* stream,
       e = cudaMemcpyAsync(dt.leaf_map, lmap.data(), lmap.size() * 4, cudaMemcpyHostToDevice, s);
     dt.device_bytes += lmap.size() * 4;
   }
-  if (e == cudaSuccess) e = fill_leaf_min(dt, s);
+  if (e == cudaSuccess) e = fill_item_min(dt, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // `ex` and `lmap` are locals
   if (e != cudaSuccess) {
     kgpu_tree_destroy(t);

@@ -1054,6 +1054,25 @@ __global__ void k_leaf_min(const uint8_t* __restrict__ arena, const uint2* __res
   }
 }
 
+// The subtrees of the `count` stems of one level, each the lesser of its two
+// children's.
+__global__ void k_node_min(uint32_t* __restrict__ m, uint32_t count) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+    const uint2 c = reinterpret_cast<const uint2*>(m)[count + i];
+    m[count + i] = min(c.x, c.y);
+  }
+}
+// The same for every level from `count` <= blockDim.x stems up to the root.
+__global__ void __launch_bounds__(1024) k_top_min(uint32_t* m, uint32_t count) {
+  for (; count; count /= 2) {
+    if (threadIdx.x < count) {
+      const uint32_t i = count + threadIdx.x;
+      m[i] = min(m[2 * i], m[2 * i + 1]);
+    }
+    __syncthreads();
+  }
+}
+
 inline unsigned blocks_for(uint64_t n, unsigned threads = 256) {
   const uint64_t b = (n + threads - 1) / threads;
   return unsigned(std::max<uint64_t>(1, std::min<uint64_t>(b, 148ull * 64)));
@@ -1275,8 +1294,8 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
        (e = scratch_alloc(reinterpret_cast<void**>(&dt.arena), dev_bytes + 16, s)) !=
            cudaSuccess) ||
       (e = scratch_alloc(&dt.extents, std::max<size_t>(16, leaves * 8), s)) != cudaSuccess ||
-      (e = scratch_alloc(reinterpret_cast<void**>(&dt.leaf_min),
-                         std::max<size_t>(16, leaves * 4), s)) != cudaSuccess ||
+      (e = scratch_alloc(reinterpret_cast<void**>(&dt.item_min),
+                         std::max<size_t>(16, leaves * 8), s)) != cudaSuccess ||
       (moved && (e = scratch_alloc(&dt.src_extents, std::max<size_t>(16, leaves * 8), s)) !=
                     cudaSuccess))
     return cuda_fail_b(e, "tree arrays");
@@ -1294,23 +1313,34 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
       g_launches++;
     }
   }
-  if ((e = cudaGetLastError()) != cudaSuccess || (e = fill_leaf_min(dt, s)) != cudaSuccess ||
+  if ((e = cudaGetLastError()) != cudaSuccess || (e = fill_item_min(dt, s)) != cudaSuccess ||
       (e = cudaStreamSynchronize(s)) != cudaSuccess)
     return cuda_fail_b(e, "writing the leaves");
   dt.device_bytes = std::max<size_t>(16, stem_count * sizeof(A)) + dev_bytes + 16 +
-                    leaves * (8 * (moved ? 2 : 1) + 4);
+                    leaves * 8 * (moved ? 3 : 2);
   return KGPU_OK;
 }
 
 }  // namespace
 
-cudaError_t fill_leaf_min(const DeviceTree& dt, cudaStream_t s) {
+cudaError_t fill_item_min(const DeviceTree& dt, cudaStream_t s) {
   if (dt.leaf_count == 0) return cudaSuccess;
   const unsigned grid = blocks_for(uint64_t(dt.leaf_count) * 32);
   auto run = [&](auto kern) {
     kern<<<grid, 256, 0, s>>>(dt.arena, static_cast<const uint2*>(dt.extents), dt.leaf_count,
-                              dt.leaf_min);
+                              dt.item_min + dt.leaf_count);
     g_launches++;
+    if (dt.scalar_walk()) return cudaGetLastError();
+    // subtrees, from the leaves up: a launch per level, the last ones in one block
+    uint32_t count = dt.leaf_count / 2;  // a power of two
+    for (; count > 1024; count /= 2) {
+      k_node_min<<<blocks_for(count), 256, 0, s>>>(dt.item_min, count);
+      g_launches++;
+    }
+    if (count) {
+      k_top_min<<<1, 1024, 0, s>>>(dt.item_min, count);
+      g_launches++;
+    }
     return cudaGetLastError();
   };
   const bool f64 = dt.dtype == KGPU_F64;

@@ -175,7 +175,8 @@ struct TreeView {
   const uint32_t* __restrict__ leaf_map;
   uint64_t map_min;
   uint32_t map_len;
-  const uint32_t* __restrict__ leaf_min;  // least item of each leaf
+  const uint32_t* __restrict__ leaf_min;  // least item of each leaf; of the subtree
+                                          // of Eytzinger stem i at i - leaf_count
 };
 
 // resolve_terminal_stem (orchestrator/mod.rs:183-192) for Mapped trees: the

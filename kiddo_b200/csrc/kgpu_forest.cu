@@ -64,7 +64,7 @@ void fill_views(const std::vector<kgpu_tree*>& trees, std::vector<uint8_t>& out)
     v.leaf_map = t.leaf_map;
     v.map_min = t.map_min;
     v.map_len = t.map_len;
-    v.leaf_min = t.leaf_min;
+    v.leaf_min = t.item_min + t.leaf_count;
     std::memcpy(out.data() + i * sizeof(TreeView<A>), &v, sizeof(v));
   }
 }

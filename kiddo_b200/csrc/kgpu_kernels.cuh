@@ -324,14 +324,6 @@ __device__ __forceinline__ bool refill_lanes(const Batch<A>& b, LaneFeeder& fd, 
   return __any_sync(FULL, active);
 }
 
-// Policies that can tell from a leaf's number that nothing in it can enter
-// their list (skip(tv, leaf)) save the warp its scan; the leaf still counts as
-// visited, as in the reference's walk.
-template <typename Pol, typename = void>
-struct HasSkip : std::false_type {};
-template <typename Pol>
-struct HasSkip<Pol, std::void_t<decltype(Pol::kSkips)>> : std::true_type {};
-
 // ---------------------------------------------------------------------------
 // The driver: lane-refilled per-thread walks, cooperative leaf scans.
 //   start(qi, tv) sets the policy up for a fresh query in this lane and says
@@ -568,7 +560,8 @@ __global__ void __launch_bounds__(256, tfixed_min_blocks<FAM, A>())
     const size_t warp0 = threadIdx.x & ~31u;
     A* lists_d = reinterpret_cast<A*>(lists);
     uint32_t* lists_i = reinterpret_cast<uint32_t*>(lists_d + size_t(k) * stride);
-    CBestN<A, K, M, EXCL> pol(lists_d + warp0 * k, lists_i + warp0 * k, nullptr, k, radius0);
+    CBestN<A, K, M, EXCL> pol(lists_d + warp0 * k, lists_i + warp0 * k, stats == nullptr, k,
+                              radius0);
     coop_drive<A, K, M>(
         tv0, b, wk, pol, slot, stride, st,
         [&](uint64_t qi, const TreeView<A>&) {
@@ -632,7 +625,7 @@ __global__ void __launch_bounds__(256) k_trow(TreeView<A> tv0, Batch<A> b, int l
   auto wk = WalkOf<A, K, M, STEMS>::make(tsmem, levels, stride);
   TravStats st;
   CRowList<A, K, M, EXCL, CartesianDist<A, K, M>> pol(best_n != 0, out_d, out_i, k,
-                                                      CartesianDist<A, K, M>());
+                                                      CartesianDist<A, K, M>(), stats == nullptr);
   coop_drive<A, K, M>(
       tv0, b, wk, pol, slot, stride, st,
       [&](uint64_t qi, const TreeView<A>&) {

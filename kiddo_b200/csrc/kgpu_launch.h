@@ -27,7 +27,9 @@ struct DeviceTree {
   // Mapped stem/leaf resolution: u32 leaf of each stem index from map_min
   // (0xffffffff: not terminal) on the device, or null (arithmetic)
   uint32_t* leaf_map = nullptr;
-  uint32_t* leaf_min = nullptr;  // least item of each leaf (0xffffffff: empty) [leaf_count]
+  // least item of each leaf (0xffffffff: empty) at [leaf_count, 2 leaf_count);
+  // below, for arithmetic Eytzinger trees, of each stem's subtree at its index
+  uint32_t* item_min = nullptr;
   uint64_t map_min = 0;
   uint32_t map_len = 0;
   // the kernels' scalar backtracking walk (Donnelly stems or Mapped resolution)
@@ -232,8 +234,8 @@ cudaError_t launch_exclusive_scan(const uint64_t* counts, uint64_t* offsets, uin
 
 int sm_count();
 
-// Fills dt.leaf_min from the stored leaves.
-cudaError_t fill_leaf_min(const DeviceTree& dt, cudaStream_t s);
+// Fills dt.item_min from the stored leaves.
+cudaError_t fill_item_min(const DeviceTree& dt, cudaStream_t s);
 
 // Re-encodes a tree's 3-D leaves between the reference's tiles (at the
 // offsets of dt.src_extents, or of dt.extents when that is null) and the

@@ -24,7 +24,7 @@ inline TreeView<A> make_view(const DeviceTree& t) {
   v.leaf_map = t.leaf_map;
   v.map_min = t.map_min;
   v.map_len = t.map_len;
-  v.leaf_min = t.leaf_min;
+  v.leaf_min = t.item_min + t.leaf_count;
   return v;
 }
 

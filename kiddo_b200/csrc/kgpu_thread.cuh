@@ -164,6 +164,15 @@ __device__ __forceinline__ uint32_t leaf_chunk_mask(const uint8_t* __restrict__ 
   return mask;
 }
 
+// Policies that can tell from a leaf's number that nothing in it can enter
+// their list (skip(tv, leaf)) save the warp its scan, the leaf still counting as
+// visited; skip_node(tv, stem) says the same of an Eytzinger subtree, which the
+// walk then passes by (never when statistics are asked for).
+template <typename Pol, typename = void>
+struct HasSkip : std::false_type {};
+template <typename Pol>
+struct HasSkip<Pol, std::void_t<decltype(Pol::kSkips)>> : std::true_type {};
+
 // Resumable traversal state of one query: the reference's DFS
 // (kd_tree/orchestrator/mod.rs:388-603) cut at its leaves, so a thread can
 // stop after any leaf and carry on later.  descend() runs from the current
@@ -229,7 +238,9 @@ struct ThreadWalk {
         pending &= ~bit;
         const A frd = slot[L * stride];
         const A md = pol.max_dist();
-        if (!(frd > md || (P::kPruneOnEqual && frd == md))) {
+        bool enter = !(frd > md || (P::kPruneOnEqual && frd == md));
+        if constexpr (HasSkip<P>::value) enter = enter && !pol.skip_node(tv, stem_idx ^ 1u);
+        if (enter) {
           const A pivot = __ldg(tv.stems + (stem_idx >> 1));
           const A old = sel(off, d);
           slot[L * stride] = old;
