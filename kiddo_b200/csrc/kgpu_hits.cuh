@@ -10,8 +10,8 @@
 // query's offset.  Records cost 20 bytes per 32 points with a hit; a batch with
 // more than its buffer holds is filled by the second walk instead.
 //
-// What bounds it: the placing pass is latency (record -> offset, query and rows
-// -> stores) hidden by four records per warp and the occupancy.
+// What bounds it: instruction issue in the counting walk; in the placing pass the
+// scattered short writes (a record's hits are about 6 words in each output).
 #pragma once
 
 #include "kgpu_kernels.cuh"
@@ -95,50 +95,57 @@ __global__ void __launch_bounds__(256) k_twithin_record(TreeView<A> tv0, Batch<A
   pol.close(lane);
 }
 
-// The records' hits at their queries' offsets: a warp takes kRecords records,
-// loads what all of them name and then writes them.
+// The records' hits at their queries' offsets.  A warp takes 32 records, a lane
+// each: the record, then its query and offset, are one load for all of them;
+// then the warp goes through the records kAhead at a time, lane p on the chunk's
+// point p.  (A warp per four records, each lane loading the same record, waited
+// on three dependent loads per four: 25M hits 506 us, 207 now.)
 template <typename A, int K, typename M>
 __global__ void __launch_bounds__(256) k_place_hits(const A* __restrict__ Q,
                                                     const uint64_t* __restrict__ offsets,
                                                     HitRecords rec, uint64_t n,
                                                     A* __restrict__ out_d,
                                                     uint32_t* __restrict__ out_i) {
-  constexpr int kRecords = 4;
+  constexpr int kAhead = 4;
   const int lane = threadIdx.x & 31;
   const uint64_t warps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
   const unsigned below_me = (1u << lane) - 1u;
-  for (uint64_t r0 = ((uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * kRecords; r0 < n;
-       r0 += warps * kRecords) {
-    uint4 leaf[kRecords];
-    uint32_t query[kRecords];
+  for (uint64_t r0 = ((uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * 32; r0 < n;
+       r0 += warps * 32) {
+    uint4 mine = make_uint4(0, 0, 0, 0);
+    uint64_t to = 0;
+    A q[K];
 #pragma unroll
-    for (int j = 0; j < kRecords; ++j) {
-      leaf[j] = make_uint4(0, 0, 0, 0);
-      query[j] = 0;
-      if (r0 + j < n) {
-        leaf[j] = __ldg(rec.leaf + r0 + j);
-        if (leaf[j].z) query[j] = __ldg(rec.query + r0 + j);
+    for (int d = 0; d < K; ++d) q[d] = A(0);
+    if (r0 + lane < n) {
+      mine = __ldg(rec.leaf + r0 + lane);
+      if (mine.z) {
+        const uint32_t query = __ldg(rec.query + r0 + lane);
+        to = __ldg(offsets + query) + mine.w;
+#pragma unroll
+        for (int d = 0; d < K; ++d) q[d] = __ldg(Q + uint64_t(query) * K + d);
       }
     }
-    A c[kRecords][K], q[kRecords][K];
-    uint32_t item[kRecords];
-    uint64_t to[kRecords];
+    for (int j0 = 0; j0 < 32; j0 += kAhead) {
+      A c[kAhead][K];
+      uint32_t item[kAhead], mask[kAhead];
 #pragma unroll
-    for (int j = 0; j < kRecords; ++j) {
-      if (!leaf[j].z) continue;
-      to[j] = __ldg(offsets + query[j]) + leaf[j].w;
+      for (int j = 0; j < kAhead; ++j) {
+        mask[j] = shfl(mine.z, j0 + j);
+        const uint64_t rows = uint64_t(shfl(mine.y, j0 + j)) << 32 | shfl(mine.x, j0 + j);
+        if ((mask[j] >> lane) & 1u)
+          load_row<A, K>(reinterpret_cast<const uint8_t*>(rows), lane, c[j], item[j]);
+      }
 #pragma unroll
-      for (int d = 0; d < K; ++d) q[j][d] = __ldg(Q + uint64_t(query[j]) * K + d);
-      const uint8_t* rows =
-          reinterpret_cast<const uint8_t*>(uint64_t(leaf[j].y) << 32 | leaf[j].x);
-      if ((leaf[j].z >> lane) & 1u) load_row<A, K>(rows, lane, c[j], item[j]);
-    }
+      for (int j = 0; j < kAhead; ++j) {
+        const uint64_t w = shfl64(to, j0 + j) + __popc(mask[j] & below_me);
+        A oq[K];
 #pragma unroll
-    for (int j = 0; j < kRecords; ++j) {
-      if ((leaf[j].z >> lane) & 1u) {
-        const uint64_t w = to[j] + __popc(leaf[j].z & below_me);
-        out_d[w] = point_dist<M, A, K>(c[j], q[j]);
-        out_i[w] = item[j];
+        for (int d = 0; d < K; ++d) oq[d] = shfl(q[d], j0 + j);
+        if ((mask[j] >> lane) & 1u) {
+          out_d[w] = point_dist<M, A, K>(c[j], oq);
+          out_i[w] = item[j];
+        }
       }
     }
   }
@@ -172,7 +179,7 @@ cudaError_t launch_place_hits(const QueryLaunch& q, const uint64_t* offsets, con
   if (n == 0) return cudaSuccess;
   return with_metric(q.metric, [&](auto m) {
     auto kern = k_place_hits<A, 3, decltype(m)>;
-    kern<<<grid_for(kern, 0, (n + 3) / 4), 256, 0, q.stream>>>(
+    kern<<<grid_for(kern, 0, (n + 31) / 32), 256, 0, q.stream>>>(
         static_cast<const A*>(q.queries), offsets, rec, n, static_cast<A*>(q.out_d), q.out_i);
     g_launches++;
     return cudaGetLastError();
