@@ -22,7 +22,7 @@ struct KeyStore;
 // the distances.  Distances are +0 or more and never NaN, so their bit patterns
 // order like their values.
 // f32: distance bits above the position in one 64-bit word.  f64: the distance
-// bits and the position.
+// and the position.
 struct KeyF32 {
   unsigned long long v;
   __device__ __forceinline__ static KeyF32 make(float d, uint32_t p) {
@@ -37,19 +37,18 @@ struct KeyF32 {
   }
 };
 struct KeyF64 {
-  unsigned long long v;
+  double d;
   uint32_t p;
-  __device__ __forceinline__ static KeyF64 make(double d, uint32_t p) {
-    return {static_cast<unsigned long long>(__double_as_longlong(d)), p};
-  }
-  __device__ __forceinline__ static KeyF64 last() { return {~0ull, ~0u}; }
+  __device__ __forceinline__ static KeyF64 make(double d, uint32_t p) { return {d, p}; }
+  __device__ __forceinline__ static KeyF64 last() { return {inf_of<double>(), ~0u}; }
+  // three chained comparisons, against six or so on the words of the two numbers
   __device__ __forceinline__ bool operator<(const KeyF64& o) const {
-    return v < o.v || (v == o.v && p < o.p);
+    return d < o.d || (d == o.d && p < o.p);
   }
-  __device__ __forceinline__ double dist() const { return __longlong_as_double((long long)v); }
+  __device__ __forceinline__ double dist() const { return d; }
   __device__ __forceinline__ uint32_t pos() const { return p; }
   __device__ __forceinline__ KeyF64 from_lane(int mask) const {
-    return {__shfl_xor_sync(FULL, v, mask), __shfl_xor_sync(FULL, p, mask)};
+    return {__shfl_xor_sync(FULL, d, mask), __shfl_xor_sync(FULL, p, mask)};
   }
 };
 template <typename A>
@@ -69,19 +68,19 @@ struct KeyStore<KeyF32> {
 };
 template <>
 struct KeyStore<KeyF64> {
-  unsigned long long* v;
+  double* v;
   uint32_t* p;
   __host__ __device__ static constexpr size_t slots(uint32_t n) { return n + n / 16; }
   __host__ __device__ static constexpr size_t bytes(uint32_t n) { return slots(n) * 12; }
   __device__ static KeyStore at(unsigned char* m, uint32_t n) {
-    unsigned long long* v = reinterpret_cast<unsigned long long*>(m);
+    double* v = reinterpret_cast<double*>(m);
     return {v, reinterpret_cast<uint32_t*>(v + slots(n))};
   }
   __device__ __forceinline__ KeyF64 get(uint32_t i) const {
     return {v[i + (i >> 4)], p[i + (i >> 4)]};
   }
   __device__ __forceinline__ void put(uint32_t i, const KeyF64& k) {
-    v[i + (i >> 4)] = k.v;
+    v[i + (i >> 4)] = k.d;
     p[i + (i >> 4)] = k.p;
   }
 };

@@ -225,7 +225,8 @@ struct CNearestNRow {
     if (nn == k) kk = shfl(Ld, k - 1);
   }
 
-  __device__ __forceinline__ void leaf(int o, uint64_t qo, const CoopLeaf<A, K>& L, int lane) {
+  __device__ __forceinline__ void leaf(int o, uint64_t qi, const CoopLeaf<A, K>& L, int lane) {
+    const uint64_t qo = shfl64(qi, o);
     int nn = __shfl_sync(FULL, n, o);
     A kk = shfl(kth, o);
     const A orad = shfl(radius, o);
@@ -350,7 +351,8 @@ struct CRowList {
            __ldg(tv.leaf_min + (int64_t(node) - int64_t(tv.leaf_count))) >= last;
   }
 
-  __device__ __forceinline__ void leaf(int o, uint64_t qo, const CoopLeaf<A, K>& L, int lane) {
+  __device__ __forceinline__ void leaf(int o, uint64_t qi, const CoopLeaf<A, K>& L, int lane) {
+    const uint64_t qo = shfl64(qi, o);
     int nn = __shfl_sync(FULL, n, o);
     A kk = shfl(kth, o);
     uint32_t lk = shfl(last, o);

@@ -25,7 +25,7 @@ struct CWithinRecord {
   static constexpr bool kPruneOnEqual = kExclusive;
   static constexpr uint32_t kBatch = 64;
   A radius;
-  uint64_t count;
+  uint32_t count;  // a tree holds fewer than 2^32 points
   HitRecords rec;
   unsigned long long at;  // the warp's next record
   uint32_t left;          // of the room it took
@@ -34,8 +34,10 @@ struct CWithinRecord {
   __device__ __forceinline__ A max_dist() const { return radius; }
   __device__ __forceinline__ bool unbounded_start() const { return radius == inf_of<A>(); }
 
-  __device__ __forceinline__ void leaf(int o, uint64_t qo, const CoopLeaf<A, K>& L, int lane) {
-    uint64_t cnt = shfl64(count, o);
+  __device__ __forceinline__ void leaf(int o, uint64_t qi, const CoopLeaf<A, K>& L, int lane) {
+    uint32_t had = 0;  // the owner's hits so far, and its query: read for the first record
+    uint32_t query = 0;
+    bool hit = false;
     const A orad = shfl(radius, o);
     for (uint32_t c0 = 0; c0 < L.len; c0 += 32) {
       const uint32_t p = c0 + lane;
@@ -47,6 +49,11 @@ struct CWithinRecord {
       }
       const unsigned m = __ballot_sync(FULL, pass);
       if (!m) continue;
+      if (!hit) {
+        had = shfl(count, o);
+        query = shfl(uint32_t(qi), o);
+        hit = true;
+      }
       if (left == 0) {
         if (lane == 0) at = atomicAdd(rec.count, (unsigned long long)kBatch);
         at = __shfl_sync(FULL, at, 0);
@@ -54,14 +61,14 @@ struct CWithinRecord {
       }
       if (lane == 0 && at < rec.cap) {
         const uint64_t rows = reinterpret_cast<uint64_t>(L.base) + c0 * row_bytes<A>();
-        rec.leaf[at] = make_uint4(uint32_t(rows), uint32_t(rows >> 32), m, uint32_t(cnt));
-        rec.query[at] = uint32_t(qo);
+        rec.leaf[at] = make_uint4(uint32_t(rows), uint32_t(rows >> 32), m, had);
+        rec.query[at] = query;
       }
       ++at;
       --left;
-      cnt += uint64_t(__popc(m));
+      had += uint32_t(__popc(m));
     }
-    if (lane == o) count = cnt;
+    if (hit && lane == o) count = had;
   }
   // Room taken and not used is left as empty records.
   __device__ __forceinline__ void close(int lane) {
@@ -89,7 +96,7 @@ __global__ void __launch_bounds__(256) k_twithin_record(TreeView<A> tv0, Batch<A
         return true;
       },
       [&](int w, uint64_t qo) {
-        const uint64_t cnt = shfl64(pol.count, w);
+        const uint32_t cnt = shfl(pol.count, w);
         if (lane == 0) counts[qo] = cnt;
       });
   pol.close(lane);

@@ -387,7 +387,7 @@ __device__ __forceinline__ void coop_drive(const TreeView<A>& tv0, const Batch<A
     }
     for (unsigned lm = __ballot_sync(FULL, active && scan); lm; lm &= lm - 1) {
       const int o = __ffs(lm) - 1;
-      pol.leaf(o, shfl64(qi, o), coop_leaf<A, K>(o, lb, len, q), lane);
+      pol.leaf(o, qi, coop_leaf<A, K>(o, lb, len, q), lane);
     }
   }
 }
@@ -759,7 +759,7 @@ __device__ __forceinline__ void periodic_drive_impl(const TreeView<A>& tv0, cons
     }
     for (unsigned lm = __ballot_sync(FULL, active); lm; lm &= lm - 1) {
       const int o = __ffs(lm) - 1;
-      pol.leaf(o, shfl64(qi, o), coop_leaf<A, K>(o, lb, len, q), lane);
+      pol.leaf(o, qi, coop_leaf<A, K>(o, lb, len, q), lane);
     }
   }
 }
