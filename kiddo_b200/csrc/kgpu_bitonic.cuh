@@ -18,6 +18,15 @@ namespace kgpu {
 template <typename Key>
 struct KeyStore;
 
+// Words below kLastWord, the largest finite double, order like the doubles with
+// their bits (denormals included), and one comparison of those takes the place of
+// two on the halves, on a pipe that is idle here: the moves of a
+// compare-exchange keep the other one busy.
+constexpr unsigned long long kLastWord = 0x7fefffffffffffffull;
+__device__ __forceinline__ bool word_less(unsigned long long a, unsigned long long b) {
+  return __longlong_as_double((long long)a) < __longlong_as_double((long long)b);
+}
+
 // Distances with a place: unique keys, so any sort of them is a stable sort of
 // the distances.  Distances are +0 or more and never NaN, so their bit patterns
 // order like their values.
@@ -28,8 +37,8 @@ struct KeyF32 {
   __device__ __forceinline__ static KeyF32 make(float d, uint32_t p) {
     return {(static_cast<unsigned long long>(__float_as_uint(d)) << 32) | p};
   }
-  __device__ __forceinline__ static KeyF32 last() { return {~0ull}; }
-  __device__ __forceinline__ bool operator<(const KeyF32& o) const { return v < o.v; }
+  __device__ __forceinline__ static KeyF32 last() { return {kLastWord}; }
+  __device__ __forceinline__ bool operator<(const KeyF32& o) const { return word_less(v, o.v); }
   __device__ __forceinline__ float dist() const { return __uint_as_float(uint32_t(v >> 32)); }
   __device__ __forceinline__ uint32_t pos() const { return uint32_t(v); }
   __device__ __forceinline__ KeyF32 from_lane(int mask) const {
