@@ -679,7 +679,7 @@ class QueryBuilder:
         self.spatial_order = None  # None: the library decides
         self.engine = None
         self.refill = None  # idle lanes before a warp refills (None: 8 to 24 by kernel)
-        self.chunk = None   # queries handed to a warp at a time (None: 32)
+        self.chunk = None   # queries handed to a warp at a time (None: 8 to 64 by kernel)
         self.stream = None
         self.points = False
         self.want_items = True
@@ -826,7 +826,7 @@ class QueryBuilder:
         """Launch knobs of the lane-refilled kernels (kgpu_query_desc::tuning):
         refill a warp's idle lanes once `refill` (1..32) are idle, hand queries
         to a warp `chunk` (a power of two, 32..1024) at a time; None keeps the
-        defaults (8 to 24 by kernel, 32).  Same results."""
+        defaults (by kernel).  Same results."""
         if refill is not None and not 1 <= int(refill) <= 32:
             raise ValueError("refill must be 1..32")
         if chunk is not None and (int(chunk) < 32 or int(chunk) > 1024 or

@@ -162,7 +162,7 @@ template <typename A>
 cudaError_t launch_within_record(const DeviceTree& t, const QueryLaunch& q, uint64_t* counts,
                                  const HitRecords& rec) {
   const TreeView<A> tv = make_view<A>(t);
-  const Batch<A> b = make_batch<A>(q, kRefillCoop);
+  const Batch<A> b = make_batch<A>(q, kRefillCoop, kChunkRadius);
   return with_metric(q.metric, [&](auto m) {
     using M = decltype(m);
     return with_excl(q.exclusive, [&](auto ex) -> cudaError_t {

@@ -76,9 +76,13 @@ inline cudaError_t with_excl(bool e, F&& f) {
 // Chunks of 32 against 64 shorten the end of a launch, where warps wait for the
 // last chunks: best_n 8.09 to 7.47 ms, kNN8 over 16 clouds 1.95 to 1.89 ms; kNN16
 // over 16M queries, whose end is a small part, keeps 64 (30.43 ms, 30.55 at 32).
+// Radius queries, whose costs differ most, go by 8 (1M over 32 catalogues 6.48 ms
+// at 32, 6.29 at 16, 6.12 at 8; best_n 3.53, 3.80, 3.53; kNN8 2.83, 2.87, 2.90).
 constexpr int kRefillScan = 24, kRefillOne = 16, kRefillCoop = 8;
+constexpr uint32_t kChunk = 32, kChunkRadius = 8;
 template <typename A>
-inline Batch<A> make_batch(const QueryLaunch& q, int refill = kRefillScan) {
+inline Batch<A> make_batch(const QueryLaunch& q, int refill = kRefillScan,
+                           uint32_t chunk = kChunk) {
   Batch<A> b;
   b.Q = static_cast<const A*>(q.queries);
   b.order = q.order;
@@ -88,7 +92,8 @@ inline Batch<A> make_batch(const QueryLaunch& q, int refill = kRefillScan) {
   b.n_trees = q.n_trees;
   b.radii = static_cast<const A*>(q.radii);
   b.work = q.work;
-  b.chunk = q.chunk ? q.chunk : refill == kRefillScan && q.nq >= (uint64_t(1) << 23) ? 64 : 32;
+  b.chunk = q.chunk ? q.chunk
+            : refill == kRefillScan && q.nq >= (uint64_t(1) << 23) ? 64 : chunk;
   b.refill = q.refill ? q.refill : refill;
   b.nq_dev = q.nq_dev;
   return b;
@@ -376,7 +381,7 @@ template <typename A, int STEMS>
 cudaError_t launch_within_pass_stems(const DeviceTree& t, const QueryLaunch& q, uint64_t* counts,
                                      const uint64_t* offsets) {
   const TreeView<A> tv = make_view<A>(t);
-  const Batch<A> b = make_batch<A>(q, kRefillCoop);
+  const Batch<A> b = make_batch<A>(q, kRefillCoop, kChunkRadius);
   const A radius = A(q.radius);
   return with_dims(t.dims, [&](auto kk) {
     constexpr int K = decltype(kk)::value;
