@@ -902,32 +902,38 @@ __global__ void k_short_rows(const uint32_t* __restrict__ counts, uint64_t n, ui
 #ifndef KGPU_HOST_SLOTS
 #define KGPU_HOST_SLOTS 3
 #endif
-#ifndef KGPU_HOST_CHUNK_LOG2
-#define KGPU_HOST_CHUNK_LOG2 19
-#endif
 #ifndef KGPU_HOST_EDGE_DIV
 #define KGPU_HOST_EDGE_DIV 8
 #endif
-// Host buffers: a batch of 2^20 queries or more goes through in chunks of 2^19
-// on three internal streams, each with its own device buffers, so the copy of
-// one chunk's queries in, another chunk's kernel and a third chunk's results out
-// run at the same time (full overlap needs pinned host memory).  With two slots a
-// chunk's kernel waited for the results of the chunk two back to leave its
-// buffers.  kNN16 (pinned, 128 result bytes a query): 2M queries 9.83 ms in one
-// piece, 8.25 in chunks of 2^18, 7.81 of 2^19; 8M queries 27.85 ms in chunks of
-// 2^21, 26.77 of 2^18, 23.03 of 2^19, against 17.9 ms for the result copy alone.
-// A smaller batch is one chunk on the caller's own stream: making streams, events
-// and a second set of buffers cost more than the overlap gave (500k queries 3.15
-// ms either way; 5,000 queries 284 us with streams and pageable results, 140
-// without and with pinned ones).  Work already queued on the caller's stream runs first; the call returns when every result is
-// on the host.
+// Queries per chunk of a host-buffer batch: two per leaf of the tree (fewer find
+// no neighbours to share leaves with), within 2^19..2^21.  kNN16, pinned, 128
+// result bytes a query: 4M-point tree (2^17 leaves) 2M queries 9.83 ms in one
+// piece, 8.25 in chunks of 2^18, 7.81 of 2^19; 8M queries 27.85 in chunks of 2^21,
+// 23.98 of 2^20, 23.22 of 2^19, against 17.9 for the result copy alone; 16M-point
+// tree (2^19 leaves), 16M queries 48.1 of 2^21, 46.7 of 2^20, 59.0 of 2^19.
+uint64_t host_chunk(const DeviceTree& dt) {
+  uint64_t c = uint64_t(1) << 19;
+  while (c < 2 * uint64_t(dt.leaf_count) && c < (uint64_t(1) << 21)) c <<= 1;
+  return c;
+}
+
+// Host buffers: a batch of two chunks or more goes through on three internal
+// streams, each with its own device buffers, so the copy of one chunk's queries
+// in, another chunk's kernel and a third chunk's results out run at the same time
+// (full overlap needs pinned host memory).  With two slots a chunk's kernel waited
+// for the results of the chunk two back to leave its buffers.  A smaller batch is
+// one chunk on the caller's own stream: making streams, events and a second set
+// of buffers cost more than the overlap gave (500k queries 3.15 ms either way;
+// 5,000 queries 284 us with streams and pageable results, 140 without and with
+// pinned ones).  Work already queued on the caller's stream runs first; the call
+// returns when every result is on the host.
 int query_host_pipelined(const DeviceTree& dt, const kgpu_query_desc* d, const QueryLaunch& base,
                          const void* queries, uint64_t nq, int w, void* out_dists,
                          uint32_t* out_items, uint32_t* out_counts, cudaStream_t s) {
   const size_t sa = dt.dtype == KGPU_F64 ? 8 : 4;
   constexpr int kSlots = KGPU_HOST_SLOTS;
-  constexpr uint64_t kChunk = uint64_t(1) << KGPU_HOST_CHUNK_LOG2;
-  const uint64_t chunk = nq < 2 * kChunk ? nq : kChunk;
+  const uint64_t full_chunk = host_chunk(dt);
+  const uint64_t chunk = nq < 2 * full_chunk ? nq : full_chunk;
   const int nslots = int(std::min<uint64_t>(kSlots, (nq + chunk - 1) / chunk));
   cudaStream_t st[kSlots] = {};
   // nearest_n without a radius fills min(k, size) entries in every row whose
