@@ -309,6 +309,8 @@ def kernel_name(fam, engine):
                 if engine != "warp" else "k_periodic_fixed<nearest_n>")
     if fam == "nearest_n" and engine == "coop":
         return "k_tnn_coop"
+    if fam == "approx" and engine != "warp":
+        return "k_approx"
     f = {"nearest_n": "nearest_n", "approx": "approx", "nearest_one": "nearest_one"}[fam]
     return f"k_tfixed<{f}>" if engine != "warp" else f"k_fixed<{f}>"
 
