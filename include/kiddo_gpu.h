@@ -374,8 +374,10 @@ int32_t kgpu_query_radius_fill(kgpu_tree* tree, const kgpu_query_desc* desc,
  * writes them from that.  Device pointers only; neither call can be captured.
  * kgpu_query_radius_count_keep waits for the total and returns it in *total
  * (offsets[nq] holds it too).  kgpu_query_radius_fill_kept takes the same
- * description, queries, offsets and stream, and `total` entries of output; it
- * may be called again.  kgpu_hits_free releases the handle after the work queued on
+ * tree, description, queries, offsets and stream, and `total` entries of output;
+ * it may be called again.  Another tree, stream or batch size is refused; with
+ * other offsets the rows are wrong, but nothing is written past a row's end or
+ * past `total`.  kgpu_hits_free releases the handle after the work queued on
  * `stream`.  A batch whose hits do not fit the handle's scratch is walked
  * again by the filling call. */
 typedef struct kgpu_hits kgpu_hits;

@@ -1182,6 +1182,7 @@ int32_t kgpu_query_radius_count_keep(kgpu_tree* t, const kgpu_query_desc* d, con
   QueryLaunch q = radius_launch(dt, d, queries, nq, s);
   auto* h = new (std::nothrow) kgpu_hits();
   if (!h) return set_error(KGPU_ENOMEM, "host allocation failed");
+  h->owner = t;
   const cudaError_t e = maybe_spatial_order(dt, d, q, h->order, h->order_tmp, s);
   h->ordered = q.order != nullptr;
   st = e == cudaSuccess ? radius_count_keep(dt, q, offsets, *h) : cuda_fail(e, "ordering the batch");
@@ -1199,7 +1200,8 @@ int32_t kgpu_query_radius_fill_kept(kgpu_tree* t, const kgpu_query_desc* d, cons
                                     void* out_dists, uint32_t* out_items, void* stream) {
   int st = check_query_desc(t, d, true);
   if (st != KGPU_OK) return st;
-  if (!hits || !offsets || hits->nq != nq) return set_error(KGPU_EINVAL, "hits of another batch");
+  if (!hits || !offsets || hits->nq != nq || hits->owner != t)
+    return set_error(KGPU_EINVAL, "hits of another batch");
   if (hits->counters.s != static_cast<cudaStream_t>(stream))
     return set_error(KGPU_EINVAL, "hits are filled on the stream that counted them");
   if (d->flags & KGPU_FLAG_HOST_BUFFERS)

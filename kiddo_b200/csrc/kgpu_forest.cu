@@ -301,6 +301,7 @@ int32_t kgpu_forest_query_radius_count_keep(kgpu_forest* f, const kgpu_query_des
   q.stream = s;
   auto* h = new (std::nothrow) kgpu_hits();
   if (!h) return set_error(KGPU_ENOMEM, "host allocation failed");
+  h->owner = f;
   DevBuf work;
   const cudaError_t e = nq ? prepare(f, d, q, work, h->order, h->order_tmp, s) : cudaSuccess;
   h->ordered = q.order != nullptr;
@@ -323,7 +324,8 @@ int32_t kgpu_forest_query_radius_fill_kept(kgpu_forest* f, const kgpu_query_desc
   QueryLaunch q;
   int st = forest_launch(f, d, queries, tree_of, radii, nq, q, true);
   if (st != KGPU_OK) return st;
-  if (!hits || !offsets || hits->nq != nq) return set_error(KGPU_EINVAL, "hits of another batch");
+  if (!hits || !offsets || hits->nq != nq || hits->owner != f)
+    return set_error(KGPU_EINVAL, "hits of another batch");
   if (hits->counters.s != static_cast<cudaStream_t>(stream))
     return set_error(KGPU_EINVAL, "hits are filled on the stream that counted them");
   if (hits->total == 0) return KGPU_OK;

@@ -5,9 +5,9 @@
 // again what the first one saw.  Here the counting pass (k_twithin_record)
 // appends a record per leaf chunk that holds hits: the chunk's address, the
 // mask of its points within the radius, the query and the hits it had before.
-// k_place_hits then takes a record per warp, recomputes the distances of the
+// k_place_hits then takes 32 records per warp, recomputes the distances of the
 // masked points (the same operations, the same bits) and writes them at the
-// query's offset.  Records cost 20 bytes per 32 points with a hit; a batch with
+// query's offset, never past the end of the query's row or of the outputs.  Records cost 20 bytes per 32 points with a hit; a batch with
 // more than its buffer holds is filled by the second walk instead.
 //
 // What bounds it: instruction issue in the counting walk; in the placing pass the
@@ -111,7 +111,7 @@ template <typename A, int K, typename M>
 __global__ void __launch_bounds__(256) k_place_hits(const A* __restrict__ Q,
                                                     const uint64_t* __restrict__ offsets,
                                                     HitRecords rec, uint64_t n,
-                                                    A* __restrict__ out_d,
+                                                    uint64_t capacity, A* __restrict__ out_d,
                                                     uint32_t* __restrict__ out_i) {
   constexpr int kAhead = 4;
   const int lane = threadIdx.x & 31;
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(256) k_place_hits(const A* __restrict__ Q,
   for (uint64_t r0 = ((uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * 32; r0 < n;
        r0 += warps * 32) {
     uint4 mine = make_uint4(0, 0, 0, 0);
-    uint64_t to = 0;
+    uint64_t to = 0, end = 0;
     A q[K];
 #pragma unroll
     for (int d = 0; d < K; ++d) q[d] = A(0);
@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(256) k_place_hits(const A* __restrict__ Q,
       if (mine.z) {
         const uint32_t query = __ldg(rec.query + r0 + lane);
         to = __ldg(offsets + query) + mine.w;
+        end = min(__ldg(offsets + query + 1), capacity);
 #pragma unroll
         for (int d = 0; d < K; ++d) q[d] = __ldg(Q + uint64_t(query) * K + d);
       }
@@ -146,10 +147,11 @@ __global__ void __launch_bounds__(256) k_place_hits(const A* __restrict__ Q,
 #pragma unroll
       for (int j = 0; j < kAhead; ++j) {
         const uint64_t w = shfl64(to, j0 + j) + __popc(mask[j] & below_me);
+        const uint64_t stop = shfl64(end, j0 + j);
         A oq[K];
 #pragma unroll
         for (int d = 0; d < K; ++d) oq[d] = shfl(q[d], j0 + j);
-        if ((mask[j] >> lane) & 1u) {
+        if (((mask[j] >> lane) & 1u) && w < stop) {
           out_d[w] = point_dist<M, A, K>(c[j], oq);
           out_i[w] = item[j];
         }
@@ -187,7 +189,8 @@ cudaError_t launch_place_hits(const QueryLaunch& q, const uint64_t* offsets, con
   return with_metric(q.metric, [&](auto m) {
     auto kern = k_place_hits<A, 3, decltype(m)>;
     kern<<<grid_for(kern, 0, (n + 31) / 32), 256, 0, q.stream>>>(
-        static_cast<const A*>(q.queries), offsets, rec, n, static_cast<A*>(q.out_d), q.out_i);
+        static_cast<const A*>(q.queries), offsets, rec, n, q.capacity, static_cast<A*>(q.out_d),
+        q.out_i);
     g_launches++;
     return cudaGetLastError();
   });

@@ -9,6 +9,7 @@
 // The processing order and, where the counting pass recorded them, the places
 // of a batch's hits; all on the stream of the counting call.
 struct kgpu_hits {
+  const void* owner = nullptr;  // the tree or forest counted; its leaves are what `rec` names
   kgpu::DevBuf order, order_tmp, leaf, query, counters;
   kgpu::HitRecords rec;
   bool ordered = false;

@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(256) k_seg_sort_small(const uint64_t* __restri
     uint64_t o = 0, n = 0;
     if (s < nq) {
       o = min(offsets[s], capacity);
-      n = min(offsets[s + 1], capacity) - o;
+      n = max(min(offsets[s + 1], capacity), o) - o;
     }
     if (n >= 2 && n <= 4) {
       small_segment_sort<A, 4>(d + o, it + o, uint32_t(n));
