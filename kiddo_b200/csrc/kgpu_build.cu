@@ -23,7 +23,10 @@
 //  * The last levels, once a node holds at most kShare points (k_finish): a
 //    block per node sorts (node, key, place) words in registers once per level
 //    and (leaf, source index, place) once more, and writes stems, leaf extents
-//    and the rows of 3-D leaves.
+//    and the rows of 3-D leaves.  Nodes that hold more than that (equal
+//    coordinates move a pivot, and shares are full where n is just below a
+//    power of two) are listed and split by the passes above for another level,
+//    until their parts fit.
 //
 // What bounds it: the level passes are HBM streams of 4 (histogram) plus 2 x
 // (4 K + 4) bytes per point and level in f32; k_finish is bound by instruction
@@ -111,7 +114,8 @@ constexpr uint64_t kTopNodes = 64;
 // it, few enough that a block's flush is small beside its points.
 inline int bins_log2_of(uint64_t nodes) { return nodes <= kTopNodes ? 13 : nodes <= 8192 ? 10 : 6; }
 
-// What one level knows of a node: its points [b, b + len), the bracket of its
+// What one level knows of a node: its number on the level, its points
+// [b, b + len), the bracket of its
 // middle (keys [klo, khi] from a sample; vlo and inv spread the values in it
 // over the inner bins), the bin of the ideal pivot, the points below and in it,
 // and how many of each kind the partition has placed.
@@ -119,14 +123,15 @@ template <typename A>
 struct Node {
   typename OrdKey<A>::U klo, khi;
   A vlo, inv;
-  uint32_t b, len;
+  uint32_t index, b, len;
   uint32_t bin, below, in;
   uint32_t placed[3];
 };
 
 template <typename A>
-__device__ __forceinline__ Node<A> new_node(uint32_t b, uint32_t len) {
+__device__ __forceinline__ Node<A> new_node(uint32_t index, uint32_t b, uint32_t len) {
   Node<A> r;
+  r.index = index;
   r.klo = r.khi = 0;
   r.vlo = r.inv = A(0);
   r.b = b;
@@ -163,11 +168,11 @@ __global__ void k_columns(const A* __restrict__ pts, uint64_t n, Columns<A, K> o
 
 template <typename A>
 __global__ void k_root(Node<A>* __restrict__ nodes, uint32_t n) {
-  nodes[0] = new_node<A>(0, n);
+  nodes[0] = new_node<A>(0, 0, n);
 }
 
-// The last node that begins at or before position p: the one holding p, as
-// empty nodes begin where the next one does.
+// The last node that begins at or before position p: the one holding p if any
+// does, as empty nodes begin where the next one does.
 template <typename A>
 __device__ __forceinline__ uint32_t node_at(const Node<A>* nodes, uint32_t count, uint32_t p) {
   uint32_t lo = 0, hi = count;
@@ -180,22 +185,21 @@ __device__ __forceinline__ uint32_t node_at(const Node<A>* nodes, uint32_t count
 }
 
 // Calls f(node, first, last) for the piece of every node inside the block's
-// share of the positions (`share` per block, in order).  Uniform in the block.
+// share of the positions (`share` per block, in order); the nodes need not cover
+// them.  Uniform in the block.
 template <typename A, typename F>
 __device__ __forceinline__ void for_each_piece(const Node<A>* nodes, uint32_t count, uint32_t n,
                                                uint32_t share, F&& f) {
   const uint64_t first = uint64_t(blockIdx.x) * share;
   if (first >= n) return;
-  uint32_t p = uint32_t(first);
+  const uint32_t p0 = uint32_t(first);
   const uint32_t end = uint32_t(first + share < n ? first + share : n);
-  uint32_t node = node_at(nodes, count, p);
-  while (p < end) {
-    const uint32_t last = min(end, nodes[node].b + nodes[node].len);
-    if (last > p) {
-      f(node, p, last);
-      p = last;
-    }
-    ++node;
+  for (uint32_t node = node_at(nodes, count, p0); node < count; ++node) {
+    const uint32_t b = nodes[node].b, stop = b + nodes[node].len;
+    if (b >= end) break;
+    const uint32_t p = max(p0, b), last = min(end, stop);
+    if (last > p) f(node, p, last);
+    if (stop >= end) break;  // spares the next node's load
   }
 }
 
@@ -639,13 +643,15 @@ __global__ void __launch_bounds__(1024) k_select(
           }
           A stem = OrdKey<A>::value(k);
           if (stem == A(0)) stem = zero_stem(cur, d, b + pivot, b + len, &zero_id);
-          if (tid == 0) stems[node] = stem;
+          if (tid == 0) stems[nodes[node].index] = stem;
         }
       }
     }
-    if (tid < 2)
+    if (tid < 2) {
+      const uint32_t child = 2 * nodes[node].index + tid;
       next[2 * uint64_t(node) + tid] =
-          tid ? new_node<A>(b + pivot, len - pivot) : new_node<A>(b, pivot);
+          tid ? new_node<A>(child, b + pivot, len - pivot) : new_node<A>(child, b, pivot);
+    }
     __syncthreads();
   }
 }
@@ -730,7 +736,7 @@ __device__ __forceinline__ void put_row(uint8_t* rows, uint32_t p, A x, A y, A z
 // remaining `levels` levels and the leaf order, all in registers and shared
 // memory.  Writes the stems, each leaf's begin and length and, in leaf order,
 // the rows of 3-D leaves (arena != null) or the source indices.  A node above
-// kShare points (equal coordinates can leave such) only raises *too_big.
+// kShare points is only counted in *too_big.
 //
 // A part of sub-level j has a slot of kShare >> j positions while every part
 // fits its slot (the parts of a split are equal but for equal coordinates), so
@@ -742,7 +748,7 @@ __global__ void __launch_bounds__(256, sizeof(A) == 4 ? 4 : 2) k_finish(
     Columns<A, K> cur, const Node<A>* __restrict__ nodes, uint32_t level,
     uint32_t levels, A* __restrict__ stems, const uint32_t* __restrict__ items,
     uint8_t* __restrict__ arena, uint32_t* __restrict__ ids, uint32_t* __restrict__ leaf_b,
-    uint32_t* __restrict__ leaf_len, int* __restrict__ too_big) {
+    uint32_t* __restrict__ leaf_len, uint32_t* __restrict__ too_big) {
   constexpr int T = 256, E = kShare / T;
   constexpr uint32_t kNone = 0xffffffffu;
   using Key = PlaceKey<A>;
@@ -752,10 +758,10 @@ __global__ void __launch_bounds__(256, sizeof(A) == 4 ? 4 : 2) k_finish(
   uint32_t* sid = reinterpret_cast<uint32_t*>(cs + size_t(K) * kShare);
   __shared__ uint32_t begin[2][65];
   __shared__ int overflow;
-  const uint32_t tid = threadIdx.x, node = blockIdx.x;
-  const uint32_t b0 = nodes[node].b, len = nodes[node].len;
+  const uint32_t tid = threadIdx.x, node = nodes[blockIdx.x].index;
+  const uint32_t b0 = nodes[blockIdx.x].b, len = nodes[blockIdx.x].len;
   if (len > kShare) {
-    if (tid == 0) *too_big = 1;
+    if (tid == 0) atomicAdd(too_big, 1u);
     return;
   }
   for (uint32_t i = tid; i < len; i += T) {
@@ -906,6 +912,29 @@ __global__ void __launch_bounds__(256, sizeof(A) == 4 ? 4 : 2) k_finish(
   }
 }
 
+// The nodes above kShare points, in order, as fresh nodes: one block.
+template <typename A>
+__global__ void __launch_bounds__(1024) k_list_big(const Node<A>* __restrict__ nodes,
+                                                   uint32_t count, Node<A>* __restrict__ out) {
+  __shared__ uint32_t warp_n[32];
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t done = 0;
+  for (uint32_t i0 = 0; i0 < count; i0 += 1024) {
+    const uint32_t i = i0 + tid;
+    const bool big = i < count && nodes[i].len > kShare;
+    const unsigned m = __ballot_sync(FULL, big);
+    if (lane == 0) warp_n[warp] = __popc(m);
+    __syncthreads();
+    uint32_t at = done + __popc(m & ((1u << lane) - 1u));
+    for (uint32_t w = 0; w < 32; ++w) {
+      at += w < warp ? warp_n[w] : 0u;
+      done += warp_n[w];
+    }
+    if (big) out[at] = new_node<A>(nodes[i].index, nodes[i].b, nodes[i].len);
+    __syncthreads();
+  }
+}
+
 // ---- leaves -------------------------------------------------------------------------
 // Encoded bytes of every leaf rounded up to 8 for the arena offsets, and the
 // longest leaf.
@@ -926,28 +955,6 @@ __global__ void k_leaf_sizes(int K, const uint32_t* __restrict__ nl, uint64_t le
   }
   longest = __reduce_max_sync(FULL, longest);
   if ((threadIdx.x & 31) == 0 && longest) atomicMax(maxlen, longest);
-}
-
-// Leaf tables and sort keys of a tree whose every level went through k_select:
-// source indices as exact double keys, segment bounds for the segment sort.
-template <typename A>
-__global__ void k_leaf_nodes(const Node<A>* __restrict__ nodes, uint64_t leaves,
-                             const uint32_t* __restrict__ id, uint64_t n,
-                             uint32_t* __restrict__ leaf_b, uint32_t* __restrict__ leaf_len,
-                             uint64_t* __restrict__ seg, double* __restrict__ keys,
-                             uint32_t* __restrict__ ids) {
-  for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n || i <= leaves;
-       i += uint64_t(gridDim.x) * blockDim.x) {
-    if (i < n) {
-      keys[i] = double(id[i]);
-      ids[i] = id[i];
-    }
-    if (i < leaves) {
-      leaf_b[i] = nodes[i].b;
-      leaf_len[i] = nodes[i].len;
-    }
-    if (i <= leaves) seg[i] = i < leaves ? nodes[i].b : n;
-  }
 }
 
 // Extents of every leaf as (offset / 8, len).  3-D rows sit at row_bytes() per
@@ -1145,16 +1152,17 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
   // top levels: those above the nodes that k_finish takes
   const uint32_t last = std::min(depth, kShareLevels), top = depth - last;
   DevBuf nodes[2], hist, lb, ll, lids, lbytes, loff, scan_tmp, flags;
-  // levels `top` and below are only reached in k_select where k_finish cannot
-  // take a node; their tables are made then
+  // A level's table holds the top levels' nodes or, below them, the parts of
+  // those that k_finish cannot take: fewer than n / kShare <= top_nodes, so
+  // their parts fill two tables' worth at most.
   const uint64_t top_nodes = uint64_t(1) << top;
   auto hist_bytes = [](uint64_t count) {  // of the levels with up to `count` nodes
     uint64_t m = 4;
     for (uint64_t c = 1; c <= count; c <<= 1) m = std::max(m, (c << bins_log2_of(c)) * 4);
     return m;
   };
-  if ((e = nodes[0].alloc(top_nodes * sizeof(Node<A>), s)) != cudaSuccess ||
-      (e = nodes[1].alloc(top_nodes * sizeof(Node<A>), s)) != cudaSuccess ||
+  if ((e = nodes[0].alloc(2 * top_nodes * sizeof(Node<A>), s)) != cudaSuccess ||
+      (e = nodes[1].alloc(2 * top_nodes * sizeof(Node<A>), s)) != cudaSuccess ||
       (e = hist.alloc(hist_bytes(top_nodes), s)) != cudaSuccess ||
       (e = lb.alloc((leaves + 1) * 4, s)) != cudaSuccess ||
       (e = ll.alloc((leaves + 1) * 4, s)) != cudaSuccess ||
@@ -1170,10 +1178,9 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
     k_root<A><<<1, 1, 0, s>>>(nodes[0].template as<Node<A>>(), uint32_t(n));
     g_launches += 2;
   }
-  // One level: the node table nodes[side] (2^level nodes) and the points in
-  // cols[cur] become the next level's.
-  auto split_level = [&](uint32_t level) -> cudaError_t {
-    const uint32_t count = 1u << level;
+  // One level: the node table nodes[side] (`count` nodes in order) and their
+  // points in cols[cur] become the next level's.
+  auto split_level = [&](uint32_t level, uint32_t count) -> cudaError_t {
     const int d = int(level % K);
     const int bins_log2 = bins_log2_of(count);
     auto* nd = nodes[side].template as<Node<A>>();
@@ -1195,7 +1202,7 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
     k_partition<A, K><<<pblocks, 256, 0, s>>>(cols[cur], cols[cur ^ 1], cols[cur].c[d], nd, count,
                                               uint32_t(n), 4096u, bins_log2);
     k_select<A, K><<<std::min(count, 148u * 16), threads, 0, s>>>(
-        cols[cur ^ 1], cols[cur], d, nd, count, stems + count,
+        cols[cur ^ 1], cols[cur], d, nd, count, stems + (uint64_t(1) << level),
         nodes[side ^ 1].template as<Node<A>>());
     g_launches += 5;
     cur ^= 1;
@@ -1203,7 +1210,8 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
     return cudaGetLastError();
   };
   for (uint32_t level = 0; level < top; ++level)
-    if ((e = split_level(level)) != cudaSuccess) return cuda_fail_b(e, "construction levels");
+    if ((e = split_level(level, 1u << level)) != cudaSuccess)
+      return cuda_fail_b(e, "construction levels");
 
   // the arena: 3-D leaves as rows, whose size is known; tiles once the leaves are
   const bool rows = RowLeaves<A, K>::value, moved = rows && sizeof(A) == 8;
@@ -1214,8 +1222,7 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
   if (rows && (e = cudaMemsetAsync(dt.arena + row_total, 0, 16, s)) != cudaSuccess)
     return cuda_fail_b(e, "arena");
   struct {
-    int too_big;
-    uint32_t max_leaf;
+    uint32_t too_big, max_leaf;
   } seen = {0, 0};
   uint64_t arena_bytes = 0;
   uint32_t last_len = 0;
@@ -1238,60 +1245,55 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
       return err;
     return cudaStreamSynchronize(s);
   };
-  DevBuf deep[2], deep_hist, lkeys, sk, si, seg;
   if (leaves) {
     auto kern = k_finish<A, K>;
     constexpr size_t smem = finish_smem<A, K>();
     if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) !=
         cudaSuccess)
       return cuda_fail_b(e, "construction");
-    // a node that k_finish leaves out leaves its leaves' lengths at 0
+    // the levels from `level` on of the `count` nodes of nodes[side] that fit
+    auto finish = [&](uint32_t level, uint32_t count) {
+      kern<<<count, 256, smem, s>>>(cols[cur], nodes[side].template as<Node<A>>(), level,
+                                    depth - level, stems, items, dt.arena, lids.as<uint32_t>(),
+                                    lb.as<uint32_t>(), ll.as<uint32_t>(), flags.as<uint32_t>());
+      g_launches++;
+      return cudaGetLastError();
+    };
+    // the leaves of nodes that k_finish leaves out have length 0 so far
     if ((e = cudaMemsetAsync(ll.p, 0, leaves * 4, s)) != cudaSuccess)
       return cuda_fail_b(e, "leaf set-up");
-    kern<<<unsigned(top_nodes), 256, smem, s>>>(
-        cols[cur], nodes[side].template as<Node<A>>(), top, last, stems, items, dt.arena,
-        lids.as<uint32_t>(), lb.as<uint32_t>(), ll.as<uint32_t>(), flags.as<int>());
-    g_launches++;
-    if ((e = cudaGetLastError()) != cudaSuccess || (e = leaf_tables()) != cudaSuccess)
+    if ((e = finish(top, uint32_t(top_nodes))) != cudaSuccess || (e = leaf_tables()) != cudaSuccess)
       return cuda_fail_b(e, "the last levels");
-    if (seen.too_big) {
-      // Equal coordinates left a node above kShare points: every remaining
-      // level by k_select, then the leaves' order by the segment sort.  The
-      // stems that k_finish wrote are written again with the same values.
-      for (int x = 0; x < 2; ++x) {
-        if ((e = deep[x].alloc(leaves * sizeof(Node<A>), s)) != cudaSuccess)
-          return cuda_fail_b(e, "construction scratch");
-      }
-      if ((e = deep_hist.alloc(hist_bytes(leaves), s)) != cudaSuccess ||
-          (e = cudaMemcpyAsync(deep[side].p, nodes[side].p, top_nodes * sizeof(Node<A>),
-                               cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
-        return cuda_fail_b(e, "construction scratch");
-      for (int x = 0; x < 2; ++x) std::swap(nodes[x].p, deep[x].p);
-      std::swap(hist.p, deep_hist.p);
-      for (uint32_t level = top; level < depth; ++level)
-        if ((e = split_level(level)) != cudaSuccess) return cuda_fail_b(e, "construction levels");
-      DevBuf ids;
-      if ((e = lkeys.alloc(n * 8, s)) != cudaSuccess || (e = ids.alloc(n * 4, s)) != cudaSuccess ||
-          (e = sk.alloc(n * 8, s)) != cudaSuccess || (e = si.alloc(n * 4, s)) != cudaSuccess ||
-          (e = seg.alloc((leaves + 1) * 8, s)) != cudaSuccess)
-        return cuda_fail_b(e, "leaf scratch");
-      std::swap(lids.p, ids.p);
-      k_leaf_nodes<A><<<blocks_for(std::max(n, leaves + 1)), 256, 0, s>>>(
-          nodes[side].template as<Node<A>>(), leaves, cols[cur].id, n, lb.as<uint32_t>(),
-          ll.as<uint32_t>(), seg.as<uint64_t>(), lkeys.as<double>(), lids.as<uint32_t>());
+    // Only the nodes that do not fit go on (a random 2^24-point f32 cloud has 24
+    // of 8,192: 4.4 ms in all; 18.4 when every node went on and every leaf was
+    // sorted again).
+    bool again = false;
+    for (uint32_t level = top, count = uint32_t(top_nodes); seen.too_big && level < depth;) {
+      again = true;
+      k_list_big<A><<<1, 1024, 0, s>>>(nodes[side].template as<Node<A>>(), count,
+                                       nodes[side ^ 1].template as<Node<A>>());
       g_launches++;
-      if ((e = leaf_tables()) != cudaSuccess) return cuda_fail_b(e, "leaf sizes");
+      side ^= 1;
+      count = seen.too_big;
+      if ((e = split_level(level, count)) != cudaSuccess)
+        return cuda_fail_b(e, "construction levels");
+      ++level;
+      count *= 2;
+      if ((e = cudaMemsetAsync(flags.p, 0, 4, s)) != cudaSuccess ||
+          (e = finish(level, count)) != cudaSuccess ||
+          (e = cudaMemcpyAsync(&seen.too_big, flags.p, 4, cudaMemcpyDeviceToHost, s)) !=
+              cudaSuccess ||
+          (e = cudaStreamSynchronize(s)) != cudaSuccess)
+        return cuda_fail_b(e, "the last levels");
     }
-    if (seen.max_leaf > 1024)
+    // a node that fits nowhere is a leaf above kShare points
+    const bool overlong = seen.too_big != 0;
+    if (again && !overlong && (e = leaf_tables()) != cudaSuccess)
+      return cuda_fail_b(e, "leaf sizes");
+    if (overlong || seen.max_leaf > 1024)
       return set_error(KGPU_EOVERFLOW,
                        "a leaf holds more than 1024 points (leaf scratch capacity, "
                        "leaf_view/mod.rs:18,58-65)");
-    // sort every leaf's ids by source index (exact as double keys)
-    if (seen.too_big &&
-        (e = launch_seg_sort<double>(seg.as<uint64_t>(), leaves, n, lkeys.as<double>(),
-                                     lids.as<uint32_t>(), sk.as<double>(), si.as<uint32_t>(), s)) !=
-            cudaSuccess)
-      return cuda_fail_b(e, "sorting the leaves");
     // the last leaf's bytes were counted rounded up to 8; the host arena ends at
     // the encoded end of the last leaf
     uint64_t raw = 0, rem = last_len;
@@ -1321,7 +1323,7 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
         lb.as<uint32_t>(), ll.as<uint32_t>(), loff.as<uint64_t>(), leaves,
         static_cast<uint2*>(dt.extents), static_cast<uint2*>(dt.src_extents));
     g_launches++;
-    if (!rows || seen.too_big) {
+    if (!rows) {
       k_write_leaves<A, K><<<blocks_for(leaves * 32), 256, 0, s>>>(
           pts, items, lids.as<uint32_t>(), lb.as<uint32_t>(), static_cast<uint2*>(dt.extents),
           leaves, dt.arena);

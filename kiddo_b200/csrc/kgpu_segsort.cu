@@ -1,5 +1,5 @@
 // kgpu_segsort.cu — stable sort of every CSR segment by distance (the sorted
-// radius families; leaf order of the device construction).
+// radius families).
 //
 // A segment's entries are sorted as (distance, position) keys.  Keys are
 // unique, so any sort of them is the stable sort of the distances, as
