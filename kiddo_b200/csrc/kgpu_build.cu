@@ -19,7 +19,9 @@
 //    levels) finds the bin that holds the ideal pivot; one pass moves the points
 //    of lower bins to the front of the node, of higher bins to its end and the
 //    bin's own into the gap, and a block per node then splits the gap (a
-//    thousandth of the points) at the pivot's key.
+//    thousandth of the points) at the pivot's key.  Should a gap be too long for
+//    a block (values spread over many exponents), the levels run once more with
+//    such gaps bracketed and partitioned again, by all blocks (split_gaps).
 //  * The last levels, once a node holds at most kShare points (k_finish): a
 //    block per node sorts (node, key, place) words in registers once per level
 //    and (leaf, source index, place) once more, and writes stems, leaf extents
@@ -110,6 +112,10 @@ constexpr uint32_t kCandidates = 256;
 constexpr int kGapBinsLog2 = 10;
 constexpr uint32_t kGapBins = 1u << kGapBinsLog2;
 constexpr uint64_t kTopNodes = 64;
+// The longest gap of different keys that k_select's one block splits at once: a
+// block reads about 40 GB/s, so this many points take 100 us or so.  Most gaps are
+// a hundredth of it.
+constexpr uint32_t kLongGap = 131072;
 // Histogram bins by the level's nodes: enough that a node's gap is small beside
 // it, few enough that a block's flush is small beside its points.
 inline int bins_log2_of(uint64_t nodes) { return nodes <= kTopNodes ? 13 : nodes <= 8192 ? 10 : 6; }
@@ -120,7 +126,7 @@ inline int bins_log2_of(uint64_t nodes) { return nodes <= kTopNodes ? 13 : nodes
 // over the inner bins), the bin of the ideal pivot, the points below and in it,
 // and how many of each kind the partition has placed.
 template <typename A>
-struct Node {
+struct alignas(16) Node {
   typename OrdKey<A>::U klo, khi;
   A vlo, inv;
   uint32_t index, b, len;
@@ -143,16 +149,28 @@ __device__ __forceinline__ Node<A> new_node(uint32_t index, uint32_t b, uint32_t
 
 __device__ __forceinline__ uint32_t ideal_pivot(uint32_t len) { return (len + 1) / 2; }
 
+// The place whose key a node is split at: the ideal pivot, or `want` of it where the
+// node is another's gap.  A place of len or more splits nothing.
+__device__ __forceinline__ uint32_t wanted(const uint32_t* want, uint32_t node, uint32_t len) {
+  return want ? want[node] : ideal_pivot(len);
+}
+
 // The bin of a coordinate: the first for keys below the bracket, the last for
 // keys above it, and in between linear in the value (each operation is
-// monotone, so bins order like keys).
-template <typename A>
+// monotone, so bins order like keys).  GAP (a long gap's bracket): linear in the
+// key instead, which resolves values over many exponents.
+template <typename A, bool GAP>
 __device__ __forceinline__ uint32_t bin_of(A x, typename OrdKey<A>::U klo,
                                            typename OrdKey<A>::U khi, A vlo, A inv,
                                            uint32_t bins) {
   const auto k = OrdKey<A>::of(x);
   if (k < klo) return 0;
   if (k > khi) return bins - 1;
+  if constexpr (GAP) {
+    // half of the bins or fewer, so that the last inner bin is never passed
+    const int shift = OrdKey<A>::bits(khi - klo) - (30 - __clz(int(bins)));
+    return 1u + uint32_t((k - klo) >> (shift > 0 ? shift : 0));
+  }
   return 1u + (inv > A(0) ? min(uint32_t(mul_rn(sub_rn(x, vlo), inv)), bins - 3) : 0u);
 }
 
@@ -194,13 +212,14 @@ __device__ __forceinline__ void for_each_piece(const Node<A>* nodes, uint32_t co
   if (first >= n) return;
   const uint32_t p0 = uint32_t(first);
   const uint32_t end = uint32_t(first + share < n ? first + share : n);
-  for (uint32_t node = node_at(nodes, count, p0); node < count; ++node) {
-    const uint32_t b = nodes[node].b, stop = b + nodes[node].len;
-    if (b >= end) break;
+  uint32_t node = node_at(nodes, count, p0), stop;
+  do {
+    const uint32_t b = nodes[node].b;
+    stop = b + nodes[node].len;
     const uint32_t p = max(p0, b), last = min(end, stop);
     if (last > p) f(node, p, last);
-    if (stop >= end) break;  // spares the next node's load
-  }
+    ++node;
+  } while (stop < end && node < count);
 }
 
 // Minimum and maximum over the block (uniform result).
@@ -240,10 +259,10 @@ __device__ __forceinline__ uint32_t sample_place(uint32_t i, uint32_t b, uint32_
   return uint32_t((uint64_t(i) * len + ((uint64_t(h) * len) >> 32)) >> 8);
 }
 
-// The bracket of every node's middle, a block per node: 256 points spread over
-// the node (sample_place), ranked by counting; the bracket runs five standard
-// deviations (8) of the sample's median to either side, about a third of the
-// points.  A middle outside it only makes k_select work longer (203 us once in
+// The bracket of every node's middle (of its wanted place, in general), a block per
+// node: 256 points spread over the node (sample_place), ranked by counting; the
+// bracket runs five standard deviations (8) of the sample's median to either side,
+// about a third of the points.  A middle outside it only makes k_select work longer (203 us once in
 // 13 levels of 16M points at four deviations, against 5 to 14).  Quantiles hold
 // for any spread of the values: over the node's whole range, bins linear in the
 // key put 1/64 of the points in one bin where the range holds zero (all
@@ -252,7 +271,8 @@ __device__ __forceinline__ uint32_t sample_place(uint32_t i, uint32_t b, uint32_
 template <typename A>
 __global__ void __launch_bounds__(256) k_bracket(const A* __restrict__ col,
                                                   Node<A>* __restrict__ nodes, uint32_t count,
-                                                  uint32_t bins) {
+                                                  uint32_t bins,
+                                                  const uint32_t* __restrict__ want) {
   using U = typename OrdKey<A>::U;
   constexpr uint32_t nt = 256, half = 40;  // sample_place shares by nt
   __shared__ U key[nt];
@@ -267,8 +287,9 @@ __global__ void __launch_bounds__(256) k_bracket(const A* __restrict__ col,
       uint32_t rank = 0;
 #pragma unroll 8
       for (uint32_t i = 0; i < nt; ++i) rank += key[i] < k || (key[i] == k && i < tid) ? 1u : 0u;
-      if (rank == nt / 2 - half) ends[0] = k;
-      if (rank == nt / 2 + half) ends[1] = k;
+      const uint32_t mid = want ? uint32_t(uint64_t(want[node]) * nt / len) : nt / 2;
+      if (rank == (mid > half ? mid - half : 0u)) ends[0] = k;
+      if (rank == min(mid + half, nt - 1)) ends[1] = k;
       __syncthreads();
       if (tid == 0) {
         const A lo = OrdKey<A>::value(ends[0]), hi = OrdKey<A>::value(ends[1]);
@@ -288,7 +309,7 @@ __global__ void __launch_bounds__(256) k_bracket(const A* __restrict__ col,
 // hist[node][bin]: the node's points by the bin of their key.  16M f32 points:
 // 46 us a level, bound by the shared-memory atomics of the inner bins (80 us
 // with one load in flight per thread).
-template <typename A>
+template <typename A, bool GAP = false>
 __global__ void __launch_bounds__(256) k_histogram(
     const A* __restrict__ col, const Node<A>* __restrict__ nodes, uint32_t count, uint32_t n,
     uint32_t share, int bins_log2, uint32_t* __restrict__ hist) {
@@ -311,7 +332,7 @@ __global__ void __launch_bounds__(256) k_histogram(
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         if (r + j * 256 + threadIdx.x >= last) continue;
-        const uint32_t at = bin_of<A>(x[j], klo, khi, vlo, inv, bins);
+        const uint32_t at = bin_of<A, GAP>(x[j], klo, khi, vlo, inv, bins);
         if (at == 0) ++first;
         else if (at == bins - 1) ++final;
         else atomicAdd(sh + at, 1u);
@@ -371,10 +392,11 @@ __device__ __forceinline__ void block_find_bin(const uint32_t* counts, uint32_t 
 template <typename A>
 __global__ void __launch_bounds__(256) k_find_bin(Node<A>* __restrict__ nodes, uint32_t count,
                                                   const uint32_t* __restrict__ hist,
-                                                  uint32_t bins) {
+                                                  uint32_t bins,
+                                                  const uint32_t* __restrict__ want) {
   __shared__ uint32_t scan[16];
   for (uint32_t node = blockIdx.x; node < count; node += gridDim.x) {
-    const uint32_t len = nodes[node].len, at = ideal_pivot(len);
+    const uint32_t len = nodes[node].len, at = wanted(want, node, len);
     uint32_t bin = 0, below = 0, in = len;
     if (at < len) block_find_bin(hist + uint64_t(node) * bins, bins, at, scan, bin, below, in);
     if (threadIdx.x == 0) {
@@ -392,7 +414,7 @@ __global__ void __launch_bounds__(256) k_find_bin(Node<A>* __restrict__ nodes, u
 // the block's room from the node's counters, so each kind is written as one run
 // per block and round.  16M f32 points: 106 us a level (4.8 TB/s), 145 with each
 // load next to its ballot.
-template <typename A, int K>
+template <typename A, int K, bool GAP = false>
 __global__ void __launch_bounds__(256) k_partition(
     Columns<A, K> in, Columns<A, K> out, const A* __restrict__ col,
     Node<A>* __restrict__ nodes, uint32_t count, uint32_t n, uint32_t share, int bins_log2) {
@@ -402,7 +424,8 @@ __global__ void __launch_bounds__(256) k_partition(
   for_each_piece(nodes, count, n, share, [&](uint32_t node, uint32_t p, uint32_t last) {
     const uint32_t b = nodes[node].b, below = nodes[node].below, inside = nodes[node].in;
     const uint32_t bin = nodes[node].bin;
-    const bool split = ideal_pivot(nodes[node].len) < nodes[node].len;
+    // (only long gaps have points where they are nodes)
+    const bool split = GAP || ideal_pivot(nodes[node].len) < nodes[node].len;
     const auto klo = nodes[node].klo, khi = nodes[node].khi;
     const A vlo = nodes[node].vlo, inv = nodes[node].inv;
     for (uint32_t r = p; r < last; r += 256 * kItems) {
@@ -429,7 +452,7 @@ __global__ void __launch_bounds__(256) k_partition(
         const uint32_t i = r + (warp * kItems + j) * 32 + lane;
         uint32_t kind = 3;
         if (i < last) {
-          const uint32_t bi = bin_of<A>(x[j], klo, khi, vlo, inv, 1u << bins_log2);
+          const uint32_t bi = bin_of<A, GAP>(x[j], klo, khi, vlo, inv, 1u << bins_log2);
           kind = !split || bi == bin ? 1 : (bi < bin ? 0 : 2);
         }
         kinds |= kind << (2 * j);
@@ -474,6 +497,54 @@ __global__ void __launch_bounds__(256) k_partition(
   });
 }
 
+// Whether a node's gap holds one key only, its klo: the bin of a bracket of one key.
+template <typename A>
+__device__ __forceinline__ bool one_key(const Node<A>& node) {
+  return node.bin == 1 && node.klo == node.khi;
+}
+
+// ---- long gaps ---------------------------------------------------------------
+// The gaps above kLongGap as nodes of their own (the other nodes are left empty)
+// with the place wanted in each; *any tells whether there are such.
+template <typename A>
+__global__ void k_list_gaps(const Node<A>* __restrict__ nodes, uint32_t count,
+                            Node<A>* __restrict__ gaps, uint32_t* __restrict__ want,
+                            uint32_t* __restrict__ any) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+    const Node<A> nd = nodes[i];
+    const uint32_t ideal = ideal_pivot(nd.len);
+    const bool is_long = ideal < nd.len && nd.in > kLongGap && !one_key(nd);
+    gaps[i] = new_node<A>(nd.index, is_long ? nd.b + nd.below : nd.b, is_long ? nd.in : 0u);
+    want[i] = is_long ? ideal - nd.below : 0u;
+    if (is_long) *any = 1;
+  }
+}
+// Their partition becomes the nodes'.
+template <typename A>
+__global__ void k_take_gaps(Node<A>* __restrict__ nodes, uint32_t count,
+                            const Node<A>* __restrict__ gaps) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+    if (!gaps[i].len) continue;
+    nodes[i].below += gaps[i].below;
+    nodes[i].in = gaps[i].in;
+    nodes[i].bin = gaps[i].bin;
+    nodes[i].klo = gaps[i].klo;
+    nodes[i].khi = gaps[i].khi;
+  }
+}
+template <typename A, int K>
+__global__ void __launch_bounds__(256) k_copy_gaps(Columns<A, K> in, Columns<A, K> out,
+                                                   const Node<A>* __restrict__ gaps,
+                                                   uint32_t count, uint32_t n, uint32_t share) {
+  for_each_piece(gaps, count, n, share, [&](uint32_t, uint32_t p, uint32_t last) {
+    for (uint32_t i = p + threadIdx.x; i < last; i += blockDim.x) {
+#pragma unroll
+      for (int a = 0; a < K; ++a) out.c[a][i] = in.c[a][i];
+      out.id[i] = in.id[i];
+    }
+  });
+}
+
 // The sign of a zero stem: that of the node's first zero in source order.
 // Points [first, last) of the column; block-wide, uniform result.
 template <typename A, int K>
@@ -496,161 +567,200 @@ __device__ A zero_stem(const Columns<A, K>& cur, int d, uint32_t first, uint32_t
   return r;
 }
 
-// One block per node: finds the key at the ideal pivot among the gap (the
-// points of its bin), moves the gap's points below it to the front and above it
-// to the back, and sets the stem and the two children.  The key is found by
+// Finds the key at a node's ideal pivot among the gap (the points of its bin), moves
+// the gap's points below it to the front and above it to the back, sets the stem
+// and returns the pivot (the node's length: no split), by the whole block.  The key is found by
 // histograms of ever narrower ranges until at most kCandidates points are in
 // range, whose keys are ranked by counting; the points move once, a thread
 // holding one each, or through `tmp` (the other set of columns, free now) when
-// the gap has more points than the block threads.
+// the gap has more points than the block threads.  A gap of one key stays as it
+// is.  Where `too_long` is given, a gap above kLongGap of different keys sets it
+// and its node is left whole (and so are others, once it is set): the caller
+// starts again.
 template <typename A, int K>
-__global__ void __launch_bounds__(1024) k_select(
-    Columns<A, K> cur, Columns<A, K> tmp, int d,
-    const Node<A>* __restrict__ nodes, uint32_t count,
-    A* __restrict__ stems, Node<A>* __restrict__ next) {
+__device__ __forceinline__ uint32_t split_node(const Columns<A, K>& cur, const Columns<A, K>& tmp,
+                                               int d, const Node<A>& nd, A* __restrict__ stems,
+                                               uint32_t* __restrict__ too_long) {
   using U = typename OrdKey<A>::U;
   __shared__ U key[kCandidates];
   __shared__ uint32_t bins[kGapBins], scan[40];
   __shared__ U red[64], found_key;
-  __shared__ uint32_t found[2], placed[3], zero_id;
+  __shared__ uint32_t found[2], placed[3], zero_id, give_up;
   const uint32_t tid = threadIdx.x, nt = blockDim.x;
-  for (uint32_t node = blockIdx.x; node < count; node += gridDim.x) {
-    const uint32_t b = nodes[node].b, len = nodes[node].len;
-    uint32_t pivot = len;
-    const uint32_t ideal = ideal_pivot(len);
-    if (ideal < len) {
-      const uint32_t lo = nodes[node].below, cnt = nodes[node].in;
-      const A* gap = cur.c[d] + b + lo;
-      // r: the wanted place among the `in` points of keys [kmin, kmax]
-      uint32_t r = ideal - lo, in = cnt, before = 0;
-      U kmin = ~U(0), kmax = 0;
-      if (cnt > kCandidates) {
-#pragma unroll 4
-        for (uint32_t i = tid; i < cnt; i += nt) {
-          const U k = OrdKey<A>::of(gap[i]);
-          kmin = k < kmin ? k : kmin;
-          kmax = k > kmax ? k : kmax;
-        }
-        block_min_max(kmin, kmax, red);
-      } else {
-        kmin = 0;
-        kmax = ~U(0);
-      }
-      while (in > kCandidates && kmin != kmax) {
-        const int width = OrdKey<A>::bits(kmax - kmin);
-        const int shift = width > kGapBinsLog2 ? width - kGapBinsLog2 : 0;
-        for (uint32_t i = tid; i < kGapBins; i += nt) bins[i] = 0;
-        __syncthreads();
-#pragma unroll 4
-        for (uint32_t i = tid; i < cnt; i += nt) {
-          const U k = OrdKey<A>::of(gap[i]);
-          if (k >= kmin && k <= kmax) atomicAdd(bins + uint32_t((k - kmin) >> shift), 1u);
-        }
-        __syncthreads();
-        uint32_t bin, below;
-        block_find_bin(bins, kGapBins, r, scan, bin, below, in);
-        __syncthreads();
-        before += below;
-        r -= below;
-        kmin += U(bin) << shift;
-        const U top = kmin + ((U(1) << shift) - 1);
-        kmax = top < kmax && top >= kmin ? top : kmax;
-      }
-      U v = kmin;
-      uint32_t lt = lo + before, equals = in;  // points below v, points equal to v
-      if (kmin != kmax) {
-        // rank the candidates by counting
-        if (tid == 0) placed[0] = 0;
-        __syncthreads();
-        for (uint32_t i = tid; i < cnt; i += nt) {
-          const U k = OrdKey<A>::of(gap[i]);
-          if (k >= kmin && k <= kmax) key[atomicAdd(placed, 1u)] = k;
-        }
-        __syncthreads();
-        if (tid < in) {
-          const U k = key[tid];
-          uint32_t less = 0, same = 0;
-          for (uint32_t i = 0; i < in; ++i) {
-            less += key[i] < k ? 1u : 0u;
-            same += key[i] == k ? 1u : 0u;
-          }
-          if (less <= r && r - less < same) {  // every holder writes the same
-            found_key = k;
-            found[0] = less;
-            found[1] = same;
-          }
-        }
-        __syncthreads();
-        v = found_key;
-        lt = lo + before + found[0];
-        equals = found[1];
-      }
-      const uint32_t le = lt + equals;
-      // below v, v, above v
-      if (tid < 3) placed[tid] = 0;
+  const uint32_t b = nd.b, len = nd.len, ideal = ideal_pivot(len);
+  if (ideal >= len) return len;
+  const uint32_t lo = nd.below, cnt = nd.in;
+  const A* gap = cur.c[d] + b + lo;
+  // r: the wanted place among the `in` points of keys [kmin, kmax]
+  uint32_t r = ideal - lo, in = cnt, before = 0;
+  U kmin = 0, kmax = ~U(0);
+  if (one_key(nd)) {
+    kmin = kmax = nd.klo;
+  } else if (cnt > kCandidates) {
+    const bool check = too_long && cnt > kLongGap;
+    if (check) {
+      if (tid == 0) give_up = atomicAdd(too_long, 0u);
       __syncthreads();
-      const uint32_t start1 = lt - lo, start2 = le - lo;
-      if (cnt <= nt) {
-        A c[K];
-        uint32_t id = 0, o = 0;
-        if (tid < cnt) {
-          const U k = OrdKey<A>::of(gap[tid]);
-          const int kind = k < v ? 0 : k == v ? 1 : 2;
-          o = (kind == 0 ? 0u : kind == 1 ? start1 : start2) + atomicAdd(placed + kind, 1u);
-#pragma unroll
-          for (int a = 0; a < K; ++a) c[a] = cur.c[a][b + lo + tid];
-          id = cur.id[b + lo + tid];
-        }
-        __syncthreads();
-        if (tid < cnt) {
-#pragma unroll
-          for (int a = 0; a < K; ++a) cur.c[a][b + lo + o] = c[a];
-          cur.id[b + lo + o] = id;
-        }
-      } else {
-        for (uint32_t i = tid; i < cnt; i += nt) {
-          const U k = OrdKey<A>::of(gap[i]);
-          const int kind = k < v ? 0 : k == v ? 1 : 2;
-          const uint32_t s = b + lo + i,
-                         o = b + lo + (kind == 0 ? 0u : kind == 1 ? start1 : start2) +
-                             atomicAdd(placed + kind, 1u);
-#pragma unroll
-          for (int a = 0; a < K; ++a) tmp.c[a][o] = cur.c[a][s];
-          tmp.id[o] = cur.id[s];
-        }
-        __syncthreads();
-        for (uint32_t i = tid; i < cnt; i += nt) {
-          const uint32_t s = b + lo + i;
-#pragma unroll
-          for (int a = 0; a < K; ++a) cur.c[a][s] = tmp.c[a][s];
-          cur.id[s] = tmp.id[s];
-        }
+      if (give_up) return len;
+    }
+    kmin = ~U(0);
+    kmax = 0;
+#pragma unroll 4
+    for (uint32_t i = tid; i < cnt; i += nt) {
+      const U k = OrdKey<A>::of(gap[i]);
+      kmin = k < kmin ? k : kmin;
+      kmax = k > kmax ? k : kmax;
+    }
+    block_min_max(kmin, kmax, red);
+    if (check && kmin != kmax) {
+      if (tid == 0) *too_long = 1;
+      return len;
+    }
+  }
+  const bool moves = kmin != kmax;
+  while (in > kCandidates && kmin != kmax) {
+    const int width = OrdKey<A>::bits(kmax - kmin);
+    const int shift = width > kGapBinsLog2 ? width - kGapBinsLog2 : 0;
+    for (uint32_t i = tid; i < kGapBins; i += nt) bins[i] = 0;
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t i = tid; i < cnt; i += nt) {
+      const U k = OrdKey<A>::of(gap[i]);
+      if (k >= kmin && k <= kmax) atomicAdd(bins + uint32_t((k - kmin) >> shift), 1u);
+    }
+    __syncthreads();
+    uint32_t bin, below;
+    block_find_bin(bins, kGapBins, r, scan, bin, below, in);
+    __syncthreads();
+    before += below;
+    r -= below;
+    kmin += U(bin) << shift;
+    const U top = kmin + ((U(1) << shift) - 1);
+    kmax = top < kmax && top >= kmin ? top : kmax;
+  }
+  U v = kmin;
+  uint32_t lt = lo + before, equals = in;  // points below v, points equal to v
+  if (kmin != kmax) {
+    // rank the candidates by counting
+    if (tid == 0) placed[0] = 0;
+    __syncthreads();
+    for (uint32_t i = tid; i < cnt; i += nt) {
+      const U k = OrdKey<A>::of(gap[i]);
+      if (k >= kmin && k <= kmax) key[atomicAdd(placed, 1u)] = k;
+    }
+    __syncthreads();
+    if (tid < in) {
+      const U k = key[tid];
+      uint32_t less = 0, same = 0;
+      for (uint32_t i = 0; i < in; ++i) {
+        less += key[i] < k ? 1u : 0u;
+        same += key[i] == k ? 1u : 0u;
       }
-      __syncthreads();
-      const A value = OrdKey<A>::value(v);
-      if (value == value) {  // a NaN at the ideal pivot splits nothing
-        pivot = lt > 0 ? lt : (le >= len ? len : le);
-        if (pivot < len) {
-          U k = v;
-          if (pivot != lt) {  // the smallest key above v
-            U least = ~U(0), most = 0;
-            for (uint32_t i = b + le + tid; i < b + len; i += nt) {
-              const U kk = OrdKey<A>::of(cur.c[d][i]);
-              least = kk < least ? kk : least;
-            }
-            block_min_max(least, most, red);
-            k = least;
-          }
-          A stem = OrdKey<A>::value(k);
-          if (stem == A(0)) stem = zero_stem(cur, d, b + pivot, b + len, &zero_id);
-          if (tid == 0) stems[nodes[node].index] = stem;
-        }
+      if (less <= r && r - less < same) {  // every holder writes the same
+        found_key = k;
+        found[0] = less;
+        found[1] = same;
       }
     }
-    if (tid < 2) {
-      const uint32_t child = 2 * nodes[node].index + tid;
-      next[2 * uint64_t(node) + tid] =
-          tid ? new_node<A>(child, b + pivot, len - pivot) : new_node<A>(child, b, pivot);
+    __syncthreads();
+    v = found_key;
+    lt = lo + before + found[0];
+    equals = found[1];
+  }
+  const uint32_t le = lt + equals;
+  // below v, v, above v
+  if (tid < 3) placed[tid] = 0;
+  __syncthreads();
+  const uint32_t start1 = lt - lo, start2 = le - lo;
+  if (!moves) {
+    // all of the gap is v
+  } else if (cnt <= nt) {
+    A c[K];
+    uint32_t id = 0, o = 0;
+    if (tid < cnt) {
+      const U k = OrdKey<A>::of(gap[tid]);
+      const int kind = k < v ? 0 : k == v ? 1 : 2;
+      o = (kind == 0 ? 0u : kind == 1 ? start1 : start2) + atomicAdd(placed + kind, 1u);
+#pragma unroll
+      for (int a = 0; a < K; ++a) c[a] = cur.c[a][b + lo + tid];
+      id = cur.id[b + lo + tid];
+    }
+    __syncthreads();
+    if (tid < cnt) {
+#pragma unroll
+      for (int a = 0; a < K; ++a) cur.c[a][b + lo + o] = c[a];
+      cur.id[b + lo + o] = id;
+    }
+  } else {
+    const unsigned below_me = (1u << (tid & 31)) - 1u;
+    for (uint32_t i0 = 0; i0 < cnt; i0 += nt) {
+      const uint32_t i = i0 + tid;
+      int kind = 3;
+      if (i < cnt) {
+        const U k = OrdKey<A>::of(gap[i]);
+        kind = k < v ? 0 : k == v ? 1 : 2;
+      }
+      uint32_t o = 0;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {  // one atomic per warp and kind
+        const unsigned m = __ballot_sync(FULL, kind == j);
+        if (kind == j) {
+          const int lead = __ffs(m) - 1;
+          uint32_t at = 0;
+          if (int(tid & 31) == lead) at = atomicAdd(placed + j, uint32_t(__popc(m)));
+          at = __shfl_sync(m, at, lead);
+          o = b + lo + (j == 0 ? 0u : j == 1 ? start1 : start2) + at + __popc(m & below_me);
+        }
+      }
+      if (kind != 3) {
+        const uint32_t s = b + lo + i;
+#pragma unroll
+        for (int a = 0; a < K; ++a) tmp.c[a][o] = cur.c[a][s];
+        tmp.id[o] = cur.id[s];
+      }
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < cnt; i += nt) {
+      const uint32_t s = b + lo + i;
+#pragma unroll
+      for (int a = 0; a < K; ++a) cur.c[a][s] = tmp.c[a][s];
+      cur.id[s] = tmp.id[s];
+    }
+  }
+  __syncthreads();
+  const A value = OrdKey<A>::value(v);
+  if (value != value) return len;  // a NaN at the ideal pivot splits nothing
+  const uint32_t pivot = lt > 0 ? lt : (le >= len ? len : le);
+  if (pivot == len) return len;
+  U k = v;
+  if (pivot != lt) {  // the smallest key above v
+    U least = ~U(0), most = 0;
+    for (uint32_t i = b + le + tid; i < b + len; i += nt) {
+      const U kk = OrdKey<A>::of(cur.c[d][i]);
+      least = kk < least ? kk : least;
+    }
+    block_min_max(least, most, red);
+    k = least;
+  }
+  A stem = OrdKey<A>::value(k);
+  if (stem == A(0)) stem = zero_stem(cur, d, b + pivot, b + len, &zero_id);
+  if (tid == 0) stems[nd.index] = stem;
+  return pivot;
+}
+
+// One block per node: its split and its two children.
+template <typename A, int K>
+__global__ void __launch_bounds__(1024, 2) k_select(
+    Columns<A, K> cur, Columns<A, K> tmp, int d,
+    const Node<A>* __restrict__ nodes, uint32_t count,
+    A* __restrict__ stems, Node<A>* __restrict__ next, uint32_t* __restrict__ too_long) {
+  for (uint32_t node = blockIdx.x; node < count; node += gridDim.x) {
+    const uint32_t pivot = split_node(cur, tmp, d, nodes[node], stems, too_long);
+    if (threadIdx.x < 2) {
+      const uint32_t b = nodes[node].b, len = nodes[node].len;
+      const uint32_t child = 2 * nodes[node].index + threadIdx.x;
+      next[2 * uint64_t(node) + threadIdx.x] =
+          threadIdx.x ? new_node<A>(child, b + pivot, len - pivot) : new_node<A>(child, b, pivot);
     }
     __syncthreads();
   }
@@ -1124,18 +1234,20 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
   dt.stem_count = stem_count;
   dt.bh = 0;
 
-  // stems (+inf = no split); the tree's arrays come from the stream-ordered
-  // pool, so rebuilding a tree of similar size reuses cached memory
+  // the tree's arrays come from the stream-ordered pool, so rebuilding a tree of
+  // similar size reuses cached memory
   dt.pooled = true;
   if ((e = scratch_alloc(&dt.stems, std::max<size_t>(16, stem_count * sizeof(A)), s)) !=
       cudaSuccess)
     return cuda_fail_b(e, "stems");
   A* stems = static_cast<A*>(dt.stems);
-  if (stem_count) {
+  auto no_stems = [&] {  // +inf = no split
+    if (!stem_count) return;
     k_fill<A><<<blocks_for(stem_count), 256, 0, s>>>(stems, stem_count,
                                                      std::numeric_limits<A>::infinity());
     g_launches++;
-  }
+  };
+  no_stems();  // launched first: an idle GPU wakes up while the scratch is allocated
 
   // two sets of columns, which the level passes move the points between
   DevBuf col[2][K], idc[2];
@@ -1170,17 +1282,64 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
       (e = lbytes.alloc((leaves + 1) * 8, s)) != cudaSuccess ||
       (e = loff.alloc((leaves + 1) * 8, s)) != cudaSuccess ||
       (e = scan_tmp.alloc(scan_tmp_bytes(leaves + 1), s)) != cudaSuccess ||
-      (e = flags.alloc(8, s)) != cudaSuccess)
+      (e = flags.alloc(16, s)) != cudaSuccess)
     return cuda_fail_b(e, "construction scratch");
+  struct {
+    uint32_t too_big, max_leaf, too_long;  // as in `flags`
+  } seen = {0, 0, 0};
   int cur = 0, side = 0;  // which columns, which node table
-  if (n) {
+  // The points in source order and one node.
+  auto set_up = [&]() -> cudaError_t {
+    cur = side = 0;
     k_columns<A, K><<<blocks_for(n), 256, 0, s>>>(pts, n, cols[0]);
     k_root<A><<<1, 1, 0, s>>>(nodes[0].template as<Node<A>>(), uint32_t(n));
     g_launches += 2;
-  }
+    return cudaMemsetAsync(flags.p, 0, 16, s);
+  };
+  // The gaps above kLongGap that a level's partition left, once more through its
+  // passes, with bins by key, until none is long (each round parts the bracket's
+  // ends, so each makes a gap shorter).  The host waits for each round.  Only for
+  // values spread over many exponents: 2^24 f32 points over 115 octaves 40 ms when one
+  // block split every gap, 9.8 now, of which 4 for the first attempt.
+  DevBuf gaps, want;
+  auto split_gaps = [&](uint32_t count, int d, int bins_log2) -> cudaError_t {
+    auto* nd = nodes[side].template as<Node<A>>();
+    cudaError_t err = cudaSuccess;
+    if (!gaps.p && ((err = gaps.alloc(2 * top_nodes * sizeof(Node<A>), s)) != cudaSuccess ||
+                    (err = want.alloc(2 * top_nodes * 4, s)) != cudaSuccess))
+      return err;
+    auto* gp = gaps.template as<Node<A>>();
+    uint32_t* at = want.template as<uint32_t>();
+    const int x = cur ^ 1;  // the columns partitioned into
+    const unsigned blocks = unsigned((n + 4095) / 4096), grid = std::min(count, 148u * 32);
+    for (int round = 0; round < 12; ++round) {
+      if ((err = cudaMemsetAsync(flags.as<uint32_t>() + 2, 0, 4, s)) != cudaSuccess) return err;
+      k_list_gaps<A><<<blocks_for(count), 256, 0, s>>>(nd, count, gp, at,
+                                                       flags.as<uint32_t>() + 2);
+      ++g_launches;
+      if ((err = cudaMemcpyAsync(&seen.too_long, flags.as<uint32_t>() + 2, 4,
+                                 cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+          (err = cudaStreamSynchronize(s)) != cudaSuccess || !seen.too_long)
+        return err;
+      if ((err = cudaMemsetAsync(hist.p, 0, (uint64_t(count) << bins_log2) * 4, s)) != cudaSuccess)
+        return err;
+      k_bracket<A><<<grid, 256, 0, s>>>(cols[x].c[d], gp, count, 1u << bins_log2, at);
+      k_histogram<A, true><<<blocks, 256, (size_t(1) << bins_log2) * 4, s>>>(
+          cols[x].c[d], gp, count, uint32_t(n), 4096u, bins_log2, hist.template as<uint32_t>());
+      k_find_bin<A><<<grid, 256, 0, s>>>(gp, count, hist.template as<uint32_t>(), 1u << bins_log2,
+                                         at);
+      k_partition<A, K, true><<<blocks, 256, 0, s>>>(cols[x], cols[cur], cols[x].c[d], gp, count,
+                                                     uint32_t(n), 4096u, bins_log2);
+      k_copy_gaps<A, K><<<blocks, 256, 0, s>>>(cols[cur], cols[x], gp, count, uint32_t(n), 4096u);
+      k_take_gaps<A><<<blocks_for(count), 256, 0, s>>>(nd, count, gp);
+      g_launches += 6;
+    }
+    return cudaGetLastError();
+  };
   // One level: the node table nodes[side] (`count` nodes in order) and their
   // points in cols[cur] become the next level's.
-  auto split_level = [&](uint32_t level, uint32_t count) -> cudaError_t {
+  // `again`: with its long gaps split by all blocks.
+  auto split_level = [&](uint32_t level, uint32_t count, bool again) -> cudaError_t {
     const int d = int(level % K);
     const int bins_log2 = bins_log2_of(count);
     auto* nd = nodes[side].template as<Node<A>>();
@@ -1193,40 +1352,32 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
     const unsigned blocks = unsigned((n + share - 1) / share);
     const int threads = count <= kTopNodes ? 1024 : 256;
     k_bracket<A><<<std::min(count, 148u * 32), 256, 0, s>>>(cols[cur].c[d], nd, count,
-                                                               1u << bins_log2);
+                                                            1u << bins_log2, nullptr);
     k_histogram<A><<<blocks, 256, (size_t(1) << bins_log2) * 4, s>>>(
         cols[cur].c[d], nd, count, uint32_t(n), share, bins_log2, hist.template as<uint32_t>());
-    k_find_bin<A><<<std::min(count, 148u * 32), 256, 0, s>>>(nd, count, hist.template as<uint32_t>(),
-                                                  1u << bins_log2);
+    k_find_bin<A><<<std::min(count, 148u * 32), 256, 0, s>>>(
+        nd, count, hist.template as<uint32_t>(), 1u << bins_log2, nullptr);
     const unsigned pblocks = unsigned((n + 4095) / 4096);
     k_partition<A, K><<<pblocks, 256, 0, s>>>(cols[cur], cols[cur ^ 1], cols[cur].c[d], nd, count,
                                               uint32_t(n), 4096u, bins_log2);
+    if (again && (err = split_gaps(count, d, bins_log2)) != cudaSuccess) return err;
     k_select<A, K><<<std::min(count, 148u * 16), threads, 0, s>>>(
         cols[cur ^ 1], cols[cur], d, nd, count, stems + (uint64_t(1) << level),
-        nodes[side ^ 1].template as<Node<A>>());
+        nodes[side ^ 1].template as<Node<A>>(), again ? nullptr : flags.as<uint32_t>() + 2);
     g_launches += 5;
     cur ^= 1;
     side ^= 1;
     return cudaGetLastError();
   };
-  for (uint32_t level = 0; level < top; ++level)
-    if ((e = split_level(level, 1u << level)) != cudaSuccess)
-      return cuda_fail_b(e, "construction levels");
-
   // the arena: 3-D leaves as rows, whose size is known; tiles once the leaves are
   const bool rows = RowLeaves<A, K>::value, moved = rows && sizeof(A) == 8;
   const uint64_t row_total = rows ? n * row_bytes<A>() : 0;
-  if (rows && (e = scratch_alloc(reinterpret_cast<void**>(&dt.arena), row_total + 16, s)) !=
-                  cudaSuccess)
-    return cuda_fail_b(e, "tree arrays");
-  if (rows && (e = cudaMemsetAsync(dt.arena + row_total, 0, 16, s)) != cudaSuccess)
-    return cuda_fail_b(e, "arena");
-  struct {
-    uint32_t too_big, max_leaf;
-  } seen = {0, 0};
+  auto make_rows = [&]() -> cudaError_t {
+    const cudaError_t err = scratch_alloc(reinterpret_cast<void**>(&dt.arena), row_total + 16, s);
+    return err != cudaSuccess ? err : cudaMemsetAsync(dt.arena + row_total, 0, 16, s);
+  };
   uint64_t arena_bytes = 0;
   uint32_t last_len = 0;
-  if ((e = cudaMemsetAsync(flags.p, 0, 8, s)) != cudaSuccess) return cuda_fail_b(e, "leaf set-up");
   // leaf sizes, offsets and what the host needs of them
   auto leaf_tables = [&]() -> cudaError_t {
     cudaError_t err = cudaMemsetAsync(lbytes.as<uint64_t>() + leaves, 0, 8, s);
@@ -1237,7 +1388,7 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
     g_launches++;
     if ((err = launch_exclusive_scan(lbytes.as<uint64_t>(), loff.as<uint64_t>(), leaves + 1,
                                      scan_tmp.p, s)) != cudaSuccess ||
-        (err = cudaMemcpyAsync(&seen, flags.p, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+        (err = cudaMemcpyAsync(&seen, flags.p, sizeof(seen), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (err = cudaMemcpyAsync(&arena_bytes, loff.as<uint64_t>() + leaves, 8,
                                cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (err = cudaMemcpyAsync(&last_len, ll.as<uint32_t>() + leaves - 1, 4,
@@ -1248,34 +1399,46 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
   if (leaves) {
     auto kern = k_finish<A, K>;
     constexpr size_t smem = finish_smem<A, K>();
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) !=
-        cudaSuccess)
-      return cuda_fail_b(e, "construction");
     // the levels from `level` on of the `count` nodes of nodes[side] that fit
-    auto finish = [&](uint32_t level, uint32_t count) {
+    auto finish = [&](uint32_t level, uint32_t count) -> cudaError_t {
+      const cudaError_t err =
+          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+      if (err != cudaSuccess) return err;
       kern<<<count, 256, smem, s>>>(cols[cur], nodes[side].template as<Node<A>>(), level,
                                     depth - level, stems, items, dt.arena, lids.as<uint32_t>(),
                                     lb.as<uint32_t>(), ll.as<uint32_t>(), flags.as<uint32_t>());
       g_launches++;
       return cudaGetLastError();
     };
-    // the leaves of nodes that k_finish leaves out have length 0 so far
-    if ((e = cudaMemsetAsync(ll.p, 0, leaves * 4, s)) != cudaSuccess)
-      return cuda_fail_b(e, "leaf set-up");
-    if ((e = finish(top, uint32_t(top_nodes))) != cudaSuccess || (e = leaf_tables()) != cudaSuccess)
-      return cuda_fail_b(e, "the last levels");
+    bool spread = false;  // a gap was too long: every level watches for such
+    do {
+      spread = seen.too_long != 0;
+      if (spread) no_stems();
+      // the leaves of nodes that k_finish leaves out have length 0 so far
+      if ((e = set_up()) != cudaSuccess ||
+          (e = cudaMemsetAsync(ll.p, 0, leaves * 4, s)) != cudaSuccess)
+        return cuda_fail_b(e, "construction set-up");
+      for (uint32_t level = 0; level < top; ++level)
+        if ((e = split_level(level, 1u << level, spread)) != cudaSuccess)
+          return cuda_fail_b(e, "construction levels");
+      if (rows && !dt.arena && (e = make_rows()) != cudaSuccess)
+        return cuda_fail_b(e, "tree arrays");
+      if ((e = finish(top, uint32_t(top_nodes))) != cudaSuccess ||
+          (e = leaf_tables()) != cudaSuccess)
+        return cuda_fail_b(e, "the last levels");
+    } while (seen.too_long && !spread);
     // Only the nodes that do not fit go on (a random 2^24-point f32 cloud has 24
     // of 8,192: 4.4 ms in all; 18.4 when every node went on and every leaf was
     // sorted again).
-    bool again = false;
+    bool more = false;
     for (uint32_t level = top, count = uint32_t(top_nodes); seen.too_big && level < depth;) {
-      again = true;
+      more = true;
       k_list_big<A><<<1, 1024, 0, s>>>(nodes[side].template as<Node<A>>(), count,
                                        nodes[side ^ 1].template as<Node<A>>());
       g_launches++;
       side ^= 1;
       count = seen.too_big;
-      if ((e = split_level(level, count)) != cudaSuccess)
+      if ((e = split_level(level, count, true)) != cudaSuccess)
         return cuda_fail_b(e, "construction levels");
       ++level;
       count *= 2;
@@ -1288,7 +1451,7 @@ int build_on_device(const A* pts, const uint32_t* items, uint64_t n, cudaStream_
     }
     // a node that fits nowhere is a leaf above kShare points
     const bool overlong = seen.too_big != 0;
-    if (again && !overlong && (e = leaf_tables()) != cudaSuccess)
+    if (more && !overlong && (e = leaf_tables()) != cudaSuccess)
       return cuda_fail_b(e, "leaf sizes");
     if (overlong || seen.max_leaf > 1024)
       return set_error(KGPU_EOVERFLOW,
