@@ -48,11 +48,13 @@ struct Batch {
   // when set, a device count that bounds nq (a compacted `order` list whose
   // length the host has not read)
   const unsigned long long* nq_dev = nullptr;
+  uint64_t dev_from = 0, dev_below = ~uint64_t(0);  // other device counts: not this launch's
 
   // the number of queries to process: nq, or less when nq_dev says so
   __device__ __forceinline__ uint64_t count() const {
     if (!nq_dev) return nq;
     const uint64_t m = *nq_dev;
+    if (m < dev_from || m >= dev_below) return 0;
     return m < nq ? m : nq;
   }
 

@@ -80,7 +80,8 @@ struct QueryLaunch {
   uint64_t total_leaves = 0;             // leaves of all trees (spatial order)
   const void* radii = nullptr;           // per-query radius (A), or null
   unsigned long long* work = nullptr;    // work-queue counter (zeroed), or null
-  const unsigned long long* nq_dev = nullptr;  // device count bounding nq (lane-refilled drivers)
+  const unsigned long long* nq_dev = nullptr;  // device count bounding nq
+  uint64_t dev_from = 0, dev_below = ~uint64_t(0);  // device counts this launch is for
   uint64_t capacity = ~uint64_t(0);      // fill pass: hits that fit the output
   int* status = nullptr;                 // fill pass: set to KGPU_EOVERFLOW on mismatch
   cudaStream_t stream = nullptr;

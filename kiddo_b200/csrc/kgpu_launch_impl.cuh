@@ -96,6 +96,8 @@ inline Batch<A> make_batch(const QueryLaunch& q, int refill = kRefillScan,
             : refill == kRefillScan && q.nq >= (uint64_t(1) << 23) ? 64 : chunk;
   b.refill = q.refill ? q.refill : refill;
   b.nq_dev = q.nq_dev;
+  b.dev_from = q.dev_from;
+  b.dev_below = q.dev_below;
   return b;
 }
 

@@ -228,8 +228,13 @@ bool point_bounds(const DeviceTree& dt, cudaStream_t caller) {
 // Batches below this size go straight to the periodic walk: the plain pass,
 // the check and the second launch cost more than they save there.
 constexpr uint64_t kFastMinBatch = uint64_t(1) << 16;
-// Batches up to this size answer the listed rows on the warp engine.
-constexpr uint64_t kWarpListed = uint64_t(1) << 21;
+// Listed rows from which threads answer them faster than warps, and the batches
+// below which that is not asked (they list fewer, unless their tree is tiny).  Where
+// both took the same, by the rows listed (f32; f64; 2-D and 3-D, uniform and
+// clustered, trees of 20k to 2M points): k = 2 34k; 30k, 8 37k; 31k, 16 40k; 38k, 32
+// 48k; 46k.  Half as many rows, threads / warps: 1.1 to 1.4; twice as many, 0.7 to 0.9.
+inline uint64_t listed_line(int k) { return 28672 + 576 * uint64_t(k); }
+constexpr uint64_t kAskMinBatch = uint64_t(1) << 17;
 
 template <typename A>
 cudaError_t periodic_fast(const DeviceTree& dt, const QueryLaunch& q, bool& handled) {
@@ -280,10 +285,20 @@ cudaError_t periodic_fast(const DeviceTree& dt, const QueryLaunch& q, bool& hand
   QueryLaunch qq = q;
   qq.order = list.as<uint32_t>();
   qq.nq_dev = n_listed.as<unsigned long long>();
-  // A batch this small lists too few rows to fill the GPU with threads, and a
-  // warp answers each of them in a twentieth of a thread's time (65,536 f64
-  // queries, k = 32: 2.29 ms in all with threads, 0.83 with warps).
-  if (q.nq <= kWarpListed && q.k <= kMaxK && q.engine == 0) qq.engine = 1;
+  if (q.k > kMaxK || q.engine != 0) return launch_fixed<A>(dt, qq);
+  // Few rows do not fill the GPU with threads, and a warp answers one in a
+  // twentieth of a thread's time (65,536 f64 queries, k = 32: 2.29 ms in all with
+  // threads, 0.83 with warps); many do (2M f64 queries on 100k points, k = 8: 4.5
+  // against 7.6).  Only the device knows how many there are: both are launched, and
+  // the one that is not meant finds no rows (5 us).
+  if (q.nq < kAskMinBatch) {
+    qq.engine = 1;
+    return launch_fixed<A>(dt, qq);
+  }
+  QueryLaunch few = qq;
+  few.engine = 1;
+  few.dev_below = qq.dev_from = listed_line(q.k);
+  if ((e = launch_fixed<A>(dt, few)) != cudaSuccess) return e;
   return launch_fixed<A>(dt, qq);
 }
 template cudaError_t periodic_fast<float>(const DeviceTree&, const QueryLaunch&, bool&);
