@@ -701,7 +701,9 @@ struct TNearestN {
       : le(reinterpret_cast<E*>(lists) + threadIdx.x),
         li(reinterpret_cast<uint32_t*>(reinterpret_cast<A*>(lists) + size_t(k_) * s) +
            threadIdx.x),
-        stride(s), n(0), k(k_), radius(r), kth(inf_of<A>()) {}
+        stride(s), n(0), k(k_), radius(r), kth(inf_of<A>()) {
+    wait() = 0;
+  }
   __device__ __forceinline__ void reset(A r) { n = 0; radius = r; kth = inf_of<A>(); }
   __device__ __forceinline__ A max_dist() const { return (n == k && kth < radius) ? kth : radius; }
   __device__ __forceinline__ bool unbounded_start() const { return radius == inf_of<A>(); }
@@ -792,7 +794,22 @@ struct TNearestN {
   // a divergent insertion for each.  The order of the words is that of
   // (distance, arrival) unless leading bits are equal: between kept entries the
   // stable sort_held puts that right, and at the cut false is returned with
-  // nothing changed.  kNN16, 16M queries: 30.5 to 28.9 ms.
+  // nothing changed.  kNN16, 16M queries: 30.5 to 28.9 ms; short lists take fewer
+  // steps than the networks (2M queries, uniform; 0.1 lattice, without / with them,
+  // ms: k = 2 1.07 / 1.11; 1.03 / 1.22, 4 1.39 / 1.36; 1.40 / 1.60, 6 1.74 / 1.64).
+  //
+  // Tried in vain it costs a scan and the networks: lattices tie at the cut, and
+  // few points lie within a short radius (k = 8 on a lattice 2.08 ms, 2.29 when every
+  // query tried; radius of 0.3 hits 0.91, 1.20).  Neighbouring queries fare
+  // alike, so after a tie a lane adds point by point for kBackOff queries, and after
+  // a first leaf that did not fill the list for the next one.
+  static constexpr int kNetworkFrom = 6, kBackOff = 32;
+  // queries before the lane tries again; in shared memory, as the kernel has no
+  // register to spare
+  __device__ __forceinline__ static uint8_t& wait() {
+    __shared__ uint8_t w[256];
+    return w[threadIdx.x];
+  }
   __device__ __forceinline__ bool first_leaf(const float4* __restrict__ rows, uint32_t len,
                                              const CartesianQ<A, K, M>& dist, A gate) {
     uint32_t w[32], passed = 0;
@@ -889,7 +906,11 @@ struct TNearestN {
     if constexpr (RowLeaves<A, K>::value && sizeof(A) == 4) {
       if (n == 0) {
         const float4* rows = reinterpret_cast<const float4*>(base);
-        if (k <= 16 && len <= 32 && first_leaf(rows, len, dist, gate)) return len;
+        const bool network = k >= kNetworkFrom && k <= 16 && len <= 32;
+        if (network && wait() == 0) {
+          if (first_leaf(rows, len, dist, gate)) return len;
+          wait() = kBackOff;
+        }
         // A leaf reached with an empty list (every query's first): each point
         // that passes the gate is added, so one pass loads, measures and adds
         // the points in leaf order instead of marking them first.
@@ -898,6 +919,10 @@ struct TNearestN {
           const A c[K] = {v.x, v.y, v.z};
           const A d = dist(c);
           if (d <= gate) add(d, __float_as_uint(v.w));
+        }
+        if (network) {
+          const uint8_t left = wait();
+          wait() = n < k ? 1 : left ? left - 1 : 0;
         }
         return len;
       }
