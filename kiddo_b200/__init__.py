@@ -89,6 +89,18 @@ def _vp(a: np.ndarray):
     return ctypes.c_void_p(a.ctypes.data) if a is not None and a.size else None
 
 
+def _make_room(total, dtype, dev, hits):
+    """The output tensors of a radius batch that did not fit beside what the
+    counting call keeps: that and the library's cached scratch go first (`hits`
+    becomes a null handle, so the fill walks the trees again)."""
+    import torch
+    C.lib().kgpu_hits_free(hits)
+    hits.value = None
+    C.scratch_trim(dev.index or 0)
+    return (torch.empty(max(total, 1), dtype=dtype, device=dev),
+            torch.empty(max(total, 1), dtype=torch.int32, device=dev))
+
+
 def _host_array(shape, dtype):
     """Result buffer in pinned host memory when torch can provide it (the
     library then copies results back at full bus speed, and without a staging
@@ -1059,13 +1071,22 @@ class QueryBuilder:
                                                    ctypes.byref(total), ctypes.byref(hits), st))
             try:
                 total = total.value
-                dist = torch.empty(max(total, 1), dtype=tdt, device=dev)
-                items = torch.empty(max(total, 1), dtype=torch.int32, device=dev)
-                C.check(L.kgpu_query_radius_fill_kept(self.tree._h, ctypes.byref(d),
-                                                      ctypes.c_void_p(q.data_ptr()), nq,
-                                                      ctypes.c_void_p(off.data_ptr()), hits,
-                                                      ctypes.c_void_p(dist.data_ptr()),
-                                                      ctypes.c_void_p(items.data_ptr()), st))
+                try:
+                    dist = torch.empty(max(total, 1), dtype=tdt, device=dev)
+                    items = torch.empty(max(total, 1), dtype=torch.int32, device=dev)
+                except torch.OutOfMemoryError:
+                    dist, items = _make_room(total, tdt, dev, hits)
+                    C.check(L.kgpu_query_radius_fill(self.tree._h, ctypes.byref(d),
+                                                     ctypes.c_void_p(q.data_ptr()), nq,
+                                                     ctypes.c_void_p(off.data_ptr()),
+                                                     ctypes.c_void_p(dist.data_ptr()),
+                                                     ctypes.c_void_p(items.data_ptr()), st))
+                else:
+                    C.check(L.kgpu_query_radius_fill_kept(self.tree._h, ctypes.byref(d),
+                                                          ctypes.c_void_p(q.data_ptr()), nq,
+                                                          ctypes.c_void_p(off.data_ptr()), hits,
+                                                          ctypes.c_void_p(dist.data_ptr()),
+                                                          ctypes.c_void_p(items.data_ptr()), st))
             finally:
                 L.kgpu_hits_free(hits)
             return WithinResult(off, dist[:total], items[:total])
@@ -1144,11 +1165,19 @@ class ForestQueryBuilder(QueryBuilder):
                 vp(off.data_ptr()), ctypes.byref(total), ctypes.byref(hits), st))
             try:
                 total = total.value
-                dist = torch.empty(max(total, 1), dtype=tdt, device=dev)
-                items = torch.empty(max(total, 1), dtype=torch.int32, device=dev)
-                C.check(L.kgpu_forest_query_radius_fill_kept(
-                    f._h, ctypes.byref(d), vp(q.data_ptr()), vp(tof.data_ptr()), rp, nq,
-                    vp(off.data_ptr()), hits, vp(dist.data_ptr()), vp(items.data_ptr()), st))
+                try:
+                    dist = torch.empty(max(total, 1), dtype=tdt, device=dev)
+                    items = torch.empty(max(total, 1), dtype=torch.int32, device=dev)
+                except torch.OutOfMemoryError:
+                    dist, items = _make_room(total, tdt, dev, hits)
+                    C.check(L.kgpu_forest_query_radius_fill(
+                        f._h, ctypes.byref(d), vp(q.data_ptr()), vp(tof.data_ptr()), rp, nq,
+                        vp(off.data_ptr()), total, vp(dist.data_ptr()), vp(items.data_ptr()),
+                        None, st))
+                else:
+                    C.check(L.kgpu_forest_query_radius_fill_kept(
+                        f._h, ctypes.byref(d), vp(q.data_ptr()), vp(tof.data_ptr()), rp, nq,
+                        vp(off.data_ptr()), hits, vp(dist.data_ptr()), vp(items.data_ptr()), st))
             finally:
                 L.kgpu_hits_free(hits)
             return WithinResult(off, dist[:total], items[:total])

@@ -1066,8 +1066,10 @@ int query_host_pipelined(const DeviceTree& dt, const kgpu_query_desc* d, const Q
 
 // Records are kept where the leaves are rows walked by ThreadWalk: 3-D
 // arithmetic trees without a periodic box, in batches that the thread engine
-// takes.  Room for 16 records per query and what the warps take in advance, at
-// most 2^26 (1.3 GB); it goes back to the pool with the handle.
+// takes.  Room for 16 records (20 bytes each) per query and what the warps take in
+// advance, at most 2^26 (1.3 GB); it goes back to the pool with the handle, at once
+// if the records did not fit, and when the sort finds no scratch beside it.  (Asking
+// the device for its free bytes to size it takes 0.4 ms.)
 int radius_count_keep(const DeviceTree& dt, QueryLaunch& q, uint64_t* offsets, kgpu_hits& hits) {
   cudaStream_t s = q.stream;
   const uint64_t nq = q.nq;
@@ -1089,7 +1091,10 @@ int radius_count_keep(const DeviceTree& dt, QueryLaunch& q, uint64_t* offsets, k
     // without room for records the batch is walked twice
     keep = hits.leaf.alloc(hits.rec.cap * sizeof(uint4), s) == cudaSuccess &&
            hits.query.alloc(hits.rec.cap * 4, s) == cudaSuccess;
-    if (!keep) cudaGetLastError();
+    if (!keep) {
+      cudaGetLastError();
+      hits.drop_records();
+    }
     hits.rec.leaf = hits.leaf.as<uint4>();
     hits.rec.query = hits.query.as<uint32_t>();
   }
@@ -1112,6 +1117,7 @@ int radius_count_keep(const DeviceTree& dt, QueryLaunch& q, uint64_t* offsets, k
     return cuda_fail(e, "radius count");
   hits.total = seen[1];
   if (keep && seen[0] <= hits.rec.cap) hits.recorded = seen[0];
+  else hits.drop_records();
   return KGPU_OK;
 }
 
@@ -1134,9 +1140,15 @@ int radius_fill_kept(const DeviceTree& dt, QueryLaunch& q, const uint64_t* offse
   if (!q.sorted) return KGPU_OK;
   const size_t sa = f64 ? 8 : 4;
   DevBuf sd, si;
-  if ((e = sd.alloc(hits.total * sa, s)) != cudaSuccess ||
-      (e = si.alloc(hits.total * 4, s)) != cudaSuccess)
-    return set_error(KGPU_ENOMEM, "device allocation failed");
+  auto scratch = [&] {
+    return (sd.p || sd.alloc(hits.total * sa, s) == cudaSuccess) &&
+           (si.p || si.alloc(hits.total * 4, s) == cudaSuccess);
+  };
+  if (!scratch()) {
+    cudaGetLastError();
+    hits.drop_records();  // placed by now
+    if (!scratch()) return set_error(KGPU_ENOMEM, "device allocation failed");
+  }
   e = f64 ? launch_seg_sort<double>(offsets, q.nq, hits.total, static_cast<double*>(q.out_d),
                                     q.out_i, sd.as<double>(), si.as<uint32_t>(), s)
           : launch_seg_sort<float>(offsets, q.nq, hits.total, static_cast<float*>(q.out_d),
@@ -1183,7 +1195,8 @@ int32_t kgpu_query_radius_count_keep(kgpu_tree* t, const kgpu_query_desc* d, con
   auto* h = new (std::nothrow) kgpu_hits();
   if (!h) return set_error(KGPU_ENOMEM, "host allocation failed");
   h->owner = t;
-  const cudaError_t e = maybe_spatial_order(dt, d, q, h->order, h->order_tmp, s);
+  DevBuf order_tmp;
+  const cudaError_t e = maybe_spatial_order(dt, d, q, h->order, order_tmp, s);
   h->ordered = q.order != nullptr;
   st = e == cudaSuccess ? radius_count_keep(dt, q, offsets, *h) : cuda_fail(e, "ordering the batch");
   if (st != KGPU_OK) {

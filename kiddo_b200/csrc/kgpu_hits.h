@@ -10,11 +10,21 @@
 // of a batch's hits; all on the stream of the counting call.
 struct kgpu_hits {
   const void* owner = nullptr;  // the tree or forest counted; its leaves are what `rec` names
-  kgpu::DevBuf order, order_tmp, leaf, query, counters;
+  kgpu::DevBuf order, counters;
+  // The records, which a fill short of scratch gives up (it then walks again).
+  mutable kgpu::DevBuf leaf, query;
   kgpu::HitRecords rec;
   bool ordered = false;
-  uint64_t recorded = ~uint64_t(0);  // records to place; ~0: none were kept, or not all
+  mutable uint64_t recorded = ~uint64_t(0);  // records to place; ~0: none are kept
   uint64_t nq = 0, total = 0;
+
+  void drop_records() const {
+    for (kgpu::DevBuf* b : {&leaf, &query}) {
+      if (b->p) cudaFreeAsync(b->p, b->s);
+      b->p = nullptr;
+    }
+    recorded = ~uint64_t(0);
+  }
 };
 
 namespace kgpu {
