@@ -911,9 +911,12 @@ __global__ void k_short_rows(const uint32_t* __restrict__ counts, uint64_t n, ui
 // piece, 8.25 in chunks of 2^18, 7.81 of 2^19; 8M queries 27.85 in chunks of 2^21,
 // 23.98 of 2^20, 23.22 of 2^19, against 17.9 for the result copy alone; 16M-point
 // tree (2^19 leaves), 16M queries 48.1 of 2^21, 46.7 of 2^20, 59.0 of 2^19.
+// No piece is larger, whatever the tree: 20M points (2^20 leaves), 3M queries 14.4
+// ms in one piece, 13.4 in two.
+constexpr uint64_t kMaxPiece = uint64_t(1) << 21;
 uint64_t host_chunk(const DeviceTree& dt) {
   uint64_t c = uint64_t(1) << 19;
-  while (c < 2 * uint64_t(dt.leaf_count) && c < (uint64_t(1) << 21)) c <<= 1;
+  while (c < 2 * uint64_t(dt.leaf_count) && c < kMaxPiece) c <<= 1;
   return c;
 }
 
@@ -925,15 +928,18 @@ uint64_t host_chunk(const DeviceTree& dt) {
 // one chunk on the caller's own stream: making streams, events and a second set
 // of buffers cost more than the overlap gave (500k queries 3.15 ms either way;
 // 5,000 queries 284 us with streams and pageable results, 140 without and with
-// pinned ones).  Work already queued on the caller's stream runs first; the call
-// returns when every result is on the host.
+// pinned ones).  The default stream stands for the calling thread's own then, which
+// follows what is queued there but not other threads' calls (4 threads, 200k
+// queries each: 0.61 ms a call on the default stream, 0.26 on their own).  Work
+// already queued on the caller's stream runs first; the call returns when every
+// result is on the host.
 int query_host_pipelined(const DeviceTree& dt, const kgpu_query_desc* d, const QueryLaunch& base,
                          const void* queries, uint64_t nq, int w, void* out_dists,
                          uint32_t* out_items, uint32_t* out_counts, cudaStream_t s) {
   const size_t sa = dt.dtype == KGPU_F64 ? 8 : 4;
   constexpr int kSlots = KGPU_HOST_SLOTS;
   const uint64_t full_chunk = host_chunk(dt);
-  const uint64_t chunk = nq < 2 * full_chunk ? nq : full_chunk;
+  const uint64_t chunk = nq < 2 * full_chunk && nq <= kMaxPiece ? nq : full_chunk;
   const int nslots = int(std::min<uint64_t>(kSlots, (nq + chunk - 1) / chunk));
   cudaStream_t st[kSlots] = {};
   // nearest_n without a radius fills min(k, size) entries in every row whose
@@ -963,7 +969,7 @@ int query_host_pipelined(const DeviceTree& dt, const kgpu_query_desc* d, const Q
   };
   cudaEvent_t ready = nullptr;
   if (nslots == 1) {
-    st[0] = s;
+    st[0] = s ? s : cudaStreamPerThread;
   } else if (e == cudaSuccess) {
     if ((e = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming)) == cudaSuccess)
       e = cudaEventRecord(ready, s);
