@@ -1,7 +1,7 @@
 """Autotuner for the query kernels.
 
 Every knob it turns leaves results bit-identical, so it only ever measures
-time.  For a (GPU, dtype, dims, family, metric, k, tree-size, periodic) key it
+time.  For a (GPU, dtype, dims, family, metric, k, tree-size, periodic, batch-size) key it
 times, on a sample of the caller's own batch, in three stages (each stage
 keeps the best choice of the ones before it):
 
@@ -65,9 +65,12 @@ def key_for(builder) -> str:
     dev = torch.cuda.get_device_name() if torch.cuda.is_available() else "cpu"
     size = tree.size() if hasattr(tree, "size") else 0
     size_bucket = int(math.log2(max(size, 1))) // 2 * 2
+    # the engines meet at some tens of thousands of queries, so a choice holds for
+    # batches within a factor of 4 only
+    batch_bucket = int(math.log2(max(len(builder.queries), 1))) // 2 * 2
     k = builder.max_qty if builder.max_qty else 1
     return "|".join(str(x) for x in (dev, tree.dtype, tree.dims, builder.family, builder.metric,
-                                     k, size_bucket, builder.box is not None))
+                                     k, size_bucket, builder.box is not None, batch_bucket))
 
 
 def engines_for(builder):
