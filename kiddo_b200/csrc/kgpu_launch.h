@@ -126,9 +126,13 @@ inline void apply_tuning(uint32_t tuning, QueryLaunch& q) {
 //     766/593; 913/632, 32768 772/798; 911/803; within f32 24576 439/441;
 //     354/308, f64 16384 567/530; 412/379
 //   f32 k = 64 49152 1164/1334; 1871/1402
-// f64 lists above 32 entries are the warp engine's at every size (49152
-// queries: k = 40 1907/1138, k = 64 3747/1719): the per-thread lists leave two
-// blocks per SM.  Explicit engines, Donnelly and Mapped trees (thread walks
+// f64 lists above 32 entries leave two blocks of threads per SM, fewer the longer
+// they are: the lines run from 65536 queries at k = 33 over 524288 at 40 to none
+// from 45 on (thread / warp engine, ms, uniform; sphere; clustered: k = 33 100k
+// queries 1.65/1.88; 1.46/1.61; 2.12/2.10, 2M 21.4/34.4; 17.1/30.0; 24.5/37.5, k =
+// 40 500k 10.8/10.8; 8.9/9.5; 12.6/12.0, 2M 38.8/41.9; 29.9/37.4; 43.4/46.4, k = 48
+// 2M 52.4/48.0; 39.4/43.2; 57.5/53.6, k = 64 2M 80.7/60.5; 58.4/54.1; 87.2/67.3).
+// Explicit engines, Donnelly and Mapped trees (thread walks
 // only) and lists kept in output rows are not touched.
 inline int engine_for(const DeviceTree& t, const QueryLaunch& q) {
   if (q.engine != 0 || t.scalar_walk() || (t.dims != 2 && t.dims != 3)) return q.engine;
@@ -142,7 +146,8 @@ inline int engine_for(const DeviceTree& t, const QueryLaunch& q) {
     case KGPU_NEAREST_N:
     case KGPU_NEAREST_N_WITHIN:
       if (q.periodic) below = k <= 32 ? (f64 ? 22528 : 28672) + 384 * k : 0;
-      else if (k > 32) below = f64 ? ~uint64_t(0) : 32768 + 512 * (k - 32);
+      else if (k > 32 && f64) below = k < 45 ? uint64_t(65536) << (k - 33) * 3 / 7 : ~uint64_t(0);
+      else if (k > 32) below = 32768 + 512 * (k - 32);
       else if (k > (f64 ? 13 : 20)) below = f64 ? 57344 : 49152;
       else below = 32768 + 768 * k;
       break;
