@@ -168,8 +168,9 @@ typedef struct kgpu_query_desc {
 } kgpu_query_desc;
 
 /* kgpu_query_desc::tuning: the lane-refilled kernels refill a warp's idle
- * lanes once n of them (1..32; default 24) are idle, and hand queries to a
- * warp 2^c at a time (c in 5..10; default 64 queries). */
+ * lanes once n of them (1..32; default 8 to 24 by kernel) are idle, and hand
+ * queries to a warp 2^c at a time (c in 5..10; default 8 to 64 queries by kernel
+ * and batch size). */
 #define KGPU_TUNE_REFILL(n) ((uint32_t)(n) & 0x3fu)
 #define KGPU_TUNE_CHUNK_LOG2(c) (((uint32_t)(c) & 0xfu) << 8)
 

@@ -257,7 +257,7 @@ __device__ __forceinline__ void flush_stats(unsigned long long* stats, const Tra
 }
 
 // Queries handed out to the lanes of one warp in chunks of Batch::chunk
-// queries (32 unless tuned): from the batch's work counter when it has one,
+// queries (8 to 64 by kernel unless tuned): from the batch's work counter when it has one,
 // else chunks gw, gw + W, gw + 2W, ... (gw = this warp, W = warps in the
 // grid).  Interleaving spreads the costly regions of a leaf-ordered batch
 // evenly over the warps.

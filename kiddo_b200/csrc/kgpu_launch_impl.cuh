@@ -74,12 +74,18 @@ inline cudaError_t with_excl(bool e, F&& f) {
 // that scan a leaf with the whole warp only idle in the walk, and refill at 8
 // (best_n over 32 catalogues, 4M queries: 7.47 ms at 24, 7.11 at 16, 7.03 at 8).
 // Chunks of 32 against 64 shorten the end of a launch, where warps wait for the
-// last chunks: best_n 8.09 to 7.47 ms, kNN8 over 16 clouds 1.95 to 1.89 ms; kNN16
-// over 16M queries, whose end is a small part, keeps 64 (30.43 ms, 30.55 at 32).
+// last chunks: best_n 8.09 to 7.47 ms, kNN8 over 16 clouds 1.95 to 1.89 ms.  Lists of
+// large batches, whose end is a small part, ask for 64 and touch the counter half as
+// often: time at 64 over time at 32 (f32 and f64, uniform and clustered, k = 4 to
+// 16) 1.05 to 1.11 at 200k queries, 1.02 to 1.08 at 1M, 0.99 to 1.01 at 4M, 0.99 to
+// 1.01 at 8M, 0.98 to 1.00 at 16M.
 // Radius queries, whose costs differ most, go by 8 (1M over 32 catalogues 6.48 ms
-// at 32, 6.29 at 16, 6.12 at 8; best_n 3.53, 3.80, 3.53; kNN8 2.83, 2.87, 2.90).
+// at 32, 6.29 at 16, 6.12 at 8; best_n 3.53, 3.80, 3.53; kNN8 2.83, 2.87, 2.90); 2-D
+// ones, whose walks are short, keep 32 (f64, 1M queries of 30 hits 2.77 ms, 2.89 at 8;
+// 300k of 300 hits 3.31, 3.55; f32 1.97, 2.03 and 2.55, 2.51).
 constexpr int kRefillScan = 24, kRefillOne = 16, kRefillCoop = 8;
-constexpr uint32_t kChunk = 32, kChunkRadius = 8;
+constexpr uint32_t kChunk = 32, kChunkRadius = 8, kChunkLarge = 64;
+constexpr uint64_t kLargeBatch = uint64_t(1) << 23;
 template <typename A>
 inline Batch<A> make_batch(const QueryLaunch& q, int refill = kRefillScan,
                            uint32_t chunk = kChunk) {
@@ -92,8 +98,7 @@ inline Batch<A> make_batch(const QueryLaunch& q, int refill = kRefillScan,
   b.n_trees = q.n_trees;
   b.radii = static_cast<const A*>(q.radii);
   b.work = q.work;
-  b.chunk = q.chunk ? q.chunk
-            : refill == kRefillScan && q.nq >= (uint64_t(1) << 23) ? 64 : chunk;
+  b.chunk = q.chunk ? q.chunk : chunk;
   b.refill = q.refill ? q.refill : refill;
   b.nq_dev = q.nq_dev;
   b.dev_from = q.dev_from;
@@ -209,9 +214,11 @@ cudaError_t launch_wfixed(const DeviceTree& t, const QueryLaunch& q) {
 template <typename A, int STEMS>
 cudaError_t launch_tfixed_stems(const DeviceTree& t, const QueryLaunch& q) {
   const TreeView<A> tv = make_view<A>(t);
+  const bool nearest = q.family == KGPU_NEAREST_N || q.family == KGPU_NEAREST_N_WITHIN;
   const Batch<A> b = make_batch<A>(
       q, q.family == KGPU_NEAREST_ONE ? kRefillOne
-                                      : q.family == KGPU_BEST_N_WITHIN ? kRefillCoop : kRefillScan);
+                                      : q.family == KGPU_BEST_N_WITHIN ? kRefillCoop : kRefillScan,
+      nearest && q.nq >= kLargeBatch ? kChunkLarge : kChunk);
   const Batch<A> coop = make_batch<A>(q, kRefillCoop);
   const A radius = A(q.radius);
   const int levels = t.max_stem_level + 2;
@@ -383,7 +390,7 @@ template <typename A, int STEMS>
 cudaError_t launch_within_pass_stems(const DeviceTree& t, const QueryLaunch& q, uint64_t* counts,
                                      const uint64_t* offsets) {
   const TreeView<A> tv = make_view<A>(t);
-  const Batch<A> b = make_batch<A>(q, kRefillCoop, kChunkRadius);
+  const Batch<A> b = make_batch<A>(q, kRefillCoop, t.dims == 3 ? kChunkRadius : kChunk);
   const A radius = A(q.radius);
   return with_dims(t.dims, [&](auto kk) {
     constexpr int K = decltype(kk)::value;
