@@ -27,9 +27,11 @@ __device__ __forceinline__ unsigned warp_first_min(double d) {
 // reports), and the first lane that holds it names the item: the first minimum
 // in leaf order, as the sequential `d < best` keeps.
 //
-// What bounds it: HBM.  Queries are taken in the caller's order, so results and
-// queries stream, and a leaf of about 30 f32 rows is one 480-byte read: 7.7 GB
-// for 16M random queries of a 16M-point tree, 1.71 ms (4.5 TB/s).  Grouping the
+// What bounds it: the latency of the leaves, half of them from HBM.  Queries are taken
+// in the caller's order, so results and queries stream, and a leaf of about 30 f32
+// rows is one 480-byte read: 7.7 GB for 16M random queries of a 16M-point clustered
+// tree, 1.71 ms, of which the L2 serves half (8M of 8M: 2.0 GB of DRAM reads, 51% of
+// issue slots, 6.9 warps waiting on loads per issue).  Grouping the
 // batch by leaf, with a leaf read once for a warp's 32 queries, took 2.72 ms:
 // 0.72 of sorting, and scattered reads of queries and writes of results.
 template <typename A, int K, typename M>

@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(256) k_find_bin(Node<A>* __restrict__ nodes, u
 // pivot's first, then the pivot's bin, then the rest.  2048 points at a time: a
 // thread holds 8, counts its warp's by kind with ballots, and one thread takes
 // the block's room from the node's counters, so each kind is written as one run
-// per block and round.  16M f32 points: 106 us a level (4.8 TB/s), 145 with each
+// per block and round.  16M f32 points: 113 us a level (4.5 TB/s), 145 with each
 // load next to its ballot.
 template <typename A, int K, bool GAP = false>
 __global__ void __launch_bounds__(256) k_partition(

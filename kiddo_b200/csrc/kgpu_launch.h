@@ -81,7 +81,7 @@ struct QueryLaunch {
   const void* radii = nullptr;           // per-query radius (A), or null
   unsigned long long* work = nullptr;    // work-queue counter (zeroed), or null
   const unsigned long long* nq_dev = nullptr;  // device count bounding nq
-  uint64_t dev_from = 0, dev_below = ~uint64_t(0);  // device counts this launch is for
+  int32_t dev_line = 0;  // device counts this launch is for (Batch::dev_line)
   uint64_t capacity = ~uint64_t(0);      // fill pass: hits that fit the output
   int* status = nullptr;                 // fill pass: set to KGPU_EOVERFLOW on mismatch
   cudaStream_t stream = nullptr;

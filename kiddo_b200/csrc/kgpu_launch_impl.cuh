@@ -101,8 +101,7 @@ inline Batch<A> make_batch(const QueryLaunch& q, int refill = kRefillScan,
   b.chunk = q.chunk ? q.chunk : chunk;
   b.refill = q.refill ? q.refill : refill;
   b.nq_dev = q.nq_dev;
-  b.dev_from = q.dev_from;
-  b.dev_below = q.dev_below;
+  b.dev_line = q.dev_line;
   return b;
 }
 

@@ -233,7 +233,7 @@ constexpr uint64_t kFastMinBatch = uint64_t(1) << 16;
 // both took the same, by the rows listed (f32; f64; 2-D and 3-D, uniform and
 // clustered, trees of 20k to 2M points): k = 2 34k; 30k, 8 37k; 31k, 16 40k; 38k, 32
 // 48k; 46k.  Half as many rows, threads / warps: 1.1 to 1.4; twice as many, 0.7 to 0.9.
-inline uint64_t listed_line(int k) { return 28672 + 576 * uint64_t(k); }
+inline int32_t listed_line(int k) { return 28672 + 576 * k; }  // k <= kMaxK
 constexpr uint64_t kAskMinBatch = uint64_t(1) << 17;
 
 template <typename A>
@@ -297,7 +297,8 @@ cudaError_t periodic_fast(const DeviceTree& dt, const QueryLaunch& q, bool& hand
   }
   QueryLaunch few = qq;
   few.engine = 1;
-  few.dev_below = qq.dev_from = listed_line(q.k);
+  qq.dev_line = listed_line(q.k);
+  few.dev_line = -qq.dev_line;
   if ((e = launch_fixed<A>(dt, few)) != cudaSuccess) return e;
   return launch_fixed<A>(dt, qq);
 }
