@@ -547,7 +547,10 @@ __global__ void __launch_bounds__(256, tfixed_min_blocks<FAM, A>())
   } else if constexpr (FAM == KF_NEAREST_N || !KGPU_BESTN_COOP) {
     // lists in shared-memory columns: entry j of thread t at j * blockDim + t
     if constexpr (FAM == KF_NEAREST_N) {
-      TNearestN<A, K, M, EXCL> pol(lists, stride, k, radius0);
+      // Of the columns of slots, Eytzinger walks leave the last one free (they use
+      // one per stem level), Donnelly walks the first (one per far child's level).
+      A* spare = STEMS ? slot : slot + size_t(levels - 1) * stride;
+      TNearestN<A, K, M, EXCL> pol(lists, stride, k, radius0, reinterpret_cast<uint32_t*>(spare));
       thread_drive<A, K, M>(tv0, b, radius0, wk, pol, slot, stride, st, [&](uint64_t qi) {
         pol.write(qi, out_d, out_i, out_c, arrival_order != 0);
       });
