@@ -1075,9 +1075,9 @@ int query_host_pipelined(const DeviceTree& dt, const kgpu_query_desc* d, const Q
 // Records are kept where the leaves are rows walked by ThreadWalk: 3-D
 // arithmetic trees without a periodic box, in batches that the thread engine
 // takes.  Room for 16 records (20 bytes each) per query and what the warps take in
-// advance, at most 2^26 (1.3 GB); it goes back to the pool with the handle, at once
-// if the records did not fit, and when the sort finds no scratch beside it.  (Asking
-// the device for its free bytes to size it takes 0.4 ms.)
+// advance, at most 2^26 (1.3 GB); it goes back to the pool with the handle, or when
+// the sort finds no scratch beside it.  (Asking the device for its free bytes to size
+// it takes 0.4 ms.)
 int radius_count_keep(const DeviceTree& dt, QueryLaunch& q, uint64_t* offsets, kgpu_hits& hits) {
   cudaStream_t s = q.stream;
   const uint64_t nq = q.nq;
@@ -1125,7 +1125,6 @@ int radius_count_keep(const DeviceTree& dt, QueryLaunch& q, uint64_t* offsets, k
     return cuda_fail(e, "radius count");
   hits.total = seen[1];
   if (keep && seen[0] <= hits.rec.cap) hits.recorded = seen[0];
-  else hits.drop_records();
   return KGPU_OK;
 }
 
@@ -1203,8 +1202,7 @@ int32_t kgpu_query_radius_count_keep(kgpu_tree* t, const kgpu_query_desc* d, con
   auto* h = new (std::nothrow) kgpu_hits();
   if (!h) return set_error(KGPU_ENOMEM, "host allocation failed");
   h->owner = t;
-  DevBuf order_tmp;
-  const cudaError_t e = maybe_spatial_order(dt, d, q, h->order, order_tmp, s);
+  const cudaError_t e = maybe_spatial_order(dt, d, q, h->order, h->order_tmp, s);
   h->ordered = q.order != nullptr;
   st = e == cudaSuccess ? radius_count_keep(dt, q, offsets, *h) : cuda_fail(e, "ordering the batch");
   if (st != KGPU_OK) {

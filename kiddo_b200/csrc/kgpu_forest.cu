@@ -302,8 +302,8 @@ int32_t kgpu_forest_query_radius_count_keep(kgpu_forest* f, const kgpu_query_des
   auto* h = new (std::nothrow) kgpu_hits();
   if (!h) return set_error(KGPU_ENOMEM, "host allocation failed");
   h->owner = f;
-  DevBuf work, order_tmp;
-  const cudaError_t e = nq ? prepare(f, d, q, work, h->order, order_tmp, s) : cudaSuccess;
+  DevBuf work;
+  const cudaError_t e = nq ? prepare(f, d, q, work, h->order, h->order_tmp, s) : cudaSuccess;
   h->ordered = q.order != nullptr;
   st = e == cudaSuccess ? radius_count_keep(f->meta, q, offsets, *h)
                         : cuda_err(e, "preparing the batch");

@@ -10,8 +10,11 @@
 // of a batch's hits; all on the stream of the counting call.
 struct kgpu_hits {
   const void* owner = nullptr;  // the tree or forest counted; its leaves are what `rec` names
-  kgpu::DevBuf order, counters;
-  // The records, which a fill short of scratch gives up (it then walks again).
+  kgpu::DevBuf order, order_tmp, counters;
+  // The records, which a fill short of scratch gives up (it then walks again).  They
+  // are not given up before, useful or not: blocks freed between the two calls
+  // leave the pool's free ranges in pieces, and the sort's scratch then waits for
+  // memory to be mapped again (90M hits 9.9 ms a call, 10 to 84 now and then).
   mutable kgpu::DevBuf leaf, query;
   kgpu::HitRecords rec;
   bool ordered = false;

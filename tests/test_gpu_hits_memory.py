@@ -1,5 +1,5 @@
-"""What a radius batch holds between counting and filling: nothing that is of no
-use, and nothing that the caller's outputs need."""
+"""What a radius batch holds between counting and filling: nothing after the
+handle is freed, and nothing that the caller's outputs need."""
 import ctypes
 
 import numpy as np
@@ -27,7 +27,7 @@ def _count_keep(tree, q, radius):
     return hits, total.value
 
 
-def test_records_that_do_not_fit_are_given_back():
+def test_a_handle_gives_everything_back():
     import torch
     rng = np.random.default_rng(12)
     n, nq = 45_000, 800                        # 1,407+ chunks a query against 16 and 2^20 in all
@@ -35,15 +35,14 @@ def test_records_that_do_not_fit_are_given_back():
     q = torch.from_numpy(rng.random((nq, 3)).astype(np.float32)).cuda()
     torch.cuda.synchronize()
     before = C.scratch_stats()[0]
-    few, total = _count_keep(tree, q, 0.001)   # records kept: 2^20 and more, 20 bytes each
-    assert total > 0 and C.scratch_stats()[0] - before > 20 << 20
-    C.lib().kgpu_hits_free(few)
-    torch.cuda.synchronize()
-    assert C.scratch_stats()[0] == before
-    many, total = _count_keep(tree, q, 4.0)    # and not kept
-    assert total == n * nq
-    assert C.scratch_stats()[0] - before < 1 << 20
-    C.lib().kgpu_hits_free(many)
+    for radius in (0.001, 4.0):                # records that fit, and that do not
+        hits, total = _count_keep(tree, q, radius)
+        assert total == n * nq if radius == 4.0 else total > 0
+        held = C.scratch_stats()[0] - before
+        assert 20 << 20 < held < 24 << 20      # 2^20 and 16 a query, 20 bytes each
+        C.lib().kgpu_hits_free(hits)
+        torch.cuda.synchronize()
+        assert C.scratch_stats()[0] == before
 
 
 @pytest.mark.parametrize("in_forest", [False, True])
