@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(256) k_place_hits(const A* __restrict__ Q,
   for (uint64_t r0 = ((uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * 32; r0 < n;
        r0 += warps * 32) {
     uint4 mine = make_uint4(0, 0, 0, 0);
-    uint64_t to = 0, end = 0;
+    uint64_t to = 0;
     A q[K];
 #pragma unroll
     for (int d = 0; d < K; ++d) q[d] = A(0);
@@ -129,7 +129,9 @@ __global__ void __launch_bounds__(256) k_place_hits(const A* __restrict__ Q,
       if (mine.z) {
         const uint32_t query = __ldg(rec.query + r0 + lane);
         to = __ldg(offsets + query) + mine.w;
-        end = min(__ldg(offsets + query + 1), capacity);
+        // a row too short for its hits keeps the first of them
+        const uint64_t end = min(__ldg(offsets + query + 1), capacity);
+        while (mine.z && to + __popc(mine.z) > end) mine.z &= ~(0x80000000u >> __clz(mine.z));
 #pragma unroll
         for (int d = 0; d < K; ++d) q[d] = __ldg(Q + uint64_t(query) * K + d);
       }
@@ -147,11 +149,10 @@ __global__ void __launch_bounds__(256) k_place_hits(const A* __restrict__ Q,
 #pragma unroll
       for (int j = 0; j < kAhead; ++j) {
         const uint64_t w = shfl64(to, j0 + j) + __popc(mask[j] & below_me);
-        const uint64_t stop = shfl64(end, j0 + j);
         A oq[K];
 #pragma unroll
         for (int d = 0; d < K; ++d) oq[d] = shfl(q[d], j0 + j);
-        if (((mask[j] >> lane) & 1u) && w < stop) {
+        if ((mask[j] >> lane) & 1u) {
           out_d[w] = point_dist<M, A, K>(c[j], oq);
           out_i[w] = item[j];
         }
